@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tc_common.cuh"
+
 namespace ew {
 
 typedef __nv_bfloat16 bf16;
@@ -28,6 +30,34 @@ __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) raw.v[i] = __float2bfloat16_rn(f[i]);
   *reinterpret_cast<Bf8*>(p) = raw;
+}
+
+// eight bf16 values in a 16-byte register group -> fp32 (a bf16 is the upper half of its fp32)
+__device__ __forceinline__ void unpack8(const uint4& r, float (&f)[8]) {
+  const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(w[i] << 16);
+    f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    w[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// e^x as __expf computes it (2^(x * log2 e) on the special-function unit), without the
+// instructions that keep subnormal results
+__device__ __forceinline__ float exp_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+  return y;
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -574,9 +604,11 @@ swiglu_bwd_kernel(const bf16* __restrict__ gu, const bf16* __restrict__ dh,
 }
 
 // ---------------------------------------------------------------------------
-// Fused softmax cross-entropy: one CTA per row of logits [rows, V] (V % 8 == 0).
+// Fused softmax cross-entropy over rows of logits [rows, V] (V % 8 == 0).
 // loss_out[row] = logsumexp - logit[target] (0 for ignored rows); the logits are
 // overwritten in place by dlogits = (softmax - onehot) * grad_scale[0].
+//
+// Any V: one CTA per row, three passes over it (maximum, sum, gradient).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(512)
 cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets,
@@ -620,6 +652,174 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ ta
       }
       store8(lr + c, f);
     }
+  }
+}
+
+// Vocabulary-sized rows.  The loop above reads a row three times from global memory and its CTAs
+// drain the memory pipe at every reduction (4096 x 32000: 159 us, 8192 x 50432: 489 us, 0.50 of
+// the copy rate).  Here a row is copied into shared memory once by a bulk copy, and two or
+// three persistent CTAs per SM work on rows of their own, so that one waits for its copy or for
+// its reduction while the others compute: with the special-function unit busy for half of the
+// time that the row's bytes take, one row at a time per SM (with the next one prefetched) came
+// to 111 / 356 us.  Measured: 104 / 330 us (5.0 TB/s, 0.76 of copy).
+constexpr int kCeThreads = 512;
+constexpr unsigned long long kCeBudgetNs = 2000000000ull;
+
+__device__ unsigned int g_ce_status;      // 1: a row's copy did not arrive within the budget
+
+struct alignas(128) CeShared {
+  float2 part[2][kCeThreads / 32];
+  uint64_t full;
+};
+
+// (maximum, sum of e^(x - maximum)) of two sets; an empty or fully masked one is (-inf, 0)
+__device__ __forceinline__ void ce_merge(float& m, float& s, float m2, float s2) {
+  const float top = fmaxf(m, m2);
+  s = (m == top ? s : s * exp_ftz(m - top)) + (m2 == top ? s2 : s2 * exp_ftz(m2 - top));
+  m = top;
+}
+
+template <int CTAS>
+__global__ void __launch_bounds__(kCeThreads, CTAS)
+cross_entropy_rows_kernel(bf16* __restrict__ logits, const long long* __restrict__ targets,
+                          float* __restrict__ loss_out, const float* __restrict__ grad_scale,
+                          int rows, int V, long long ignore_index) {
+  extern __shared__ __align__(128) uint8_t ce_smem[];
+  CeShared* sh = reinterpret_cast<CeShared*>(ce_smem);
+  const bf16* br = reinterpret_cast<const bf16*>(ce_smem + sizeof(CeShared));
+  const int tid = threadIdx.x;
+  const uint32_t row_bytes = (uint32_t)V * 2u;
+  auto load = [&](long long row) {
+    tc::mbar_expect_tx(&sh->full, row_bytes);
+    tc::bulk_load(ce_smem + sizeof(CeShared), logits + (size_t)row * V, row_bytes, &sh->full);
+  };
+  if (tid == 0) {
+    tc::mbar_init(&sh->full, 1);
+    tc::fence_mbar_init();
+    if (blockIdx.x < rows) load(blockIdx.x);
+  }
+  __syncthreads();
+
+  const int vec = V / 8;
+  const float gscale = grad_scale[0];
+  int it = 0;
+  unsigned long long budget = kCeBudgetNs;
+  long long tgt = blockIdx.x < rows ? targets[blockIdx.x] : 0;
+  for (long long row = blockIdx.x; row < rows; row += gridDim.x, ++it) {
+    // the next row's target is requested a row ahead: its latency would stall every row
+    const long long next_tgt = row + gridDim.x < rows ? targets[row + gridDim.x] : 0;
+    const bool ignored = tgt == ignore_index || tgt < 0 || tgt >= V;
+    if (!tc::mbar_wait(&sh->full, (uint32_t)it & 1u, budget)) {
+      // go on with what is there (a thread that left would leave the others in a barrier), but
+      // do not wait again
+      atomicCAS(&g_ce_status, 0u, 1u);
+      budget = 0;
+    }
+    float m = -INFINITY;
+#pragma unroll 4
+    for (int c = tid; c < vec; c += kCeThreads) {
+      float f[8];
+      unpack8(*reinterpret_cast<const uint4*>(br + c * 8), f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m = fmaxf(m, f[i]);
+    }
+    // Sum relative to the warp's own maximum, so that maximum and sum need one barrier.  A warp
+    // whose values are all -inf uses 0 instead: its sum is then 0, not NaN.
+    m = warp_max(m);
+    const float ref = m == -INFINITY ? 0.0f : m;
+    float s4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+    for (int c = tid; c < vec; c += kCeThreads) {
+      float f[8];
+      unpack8(*reinterpret_cast<const uint4*>(br + c * 8), f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s4[i & 3] += exp_ftz(f[i] - ref);
+    }
+    float s = warp_sum((s4[0] + s4[1]) + (s4[2] + s4[3]));
+    if ((tid & 31) == 0) sh->part[it & 1][tid >> 5] = make_float2(m, s);
+    __syncthreads();
+    {
+      const float2 p = sh->part[it & 1][tid & (kCeThreads / 32 - 1)];
+      m = p.x;
+      s = p.y;
+#pragma unroll
+      for (int o = kCeThreads / 64; o > 0; o >>= 1)
+        ce_merge(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
+    }
+    const float scale = ignored ? 0.0f : gscale;
+    const float factor = 1.0f / s * scale;
+    bf16* gr = logits + (size_t)row * V;
+#pragma unroll 4
+    for (int c = tid; c < vec; c += kCeThreads) {
+      float f[8];
+      unpack8(*reinterpret_cast<const uint4*>(br + c * 8), f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = exp_ftz(f[i] - m) * factor;
+      *reinterpret_cast<uint4*>(gr + c * 8) = pack8(f);
+    }
+    // The target's own element is written once more by the thread that owns its group: a test
+    // in the loop would make the compiler index the group through local memory.
+    if (!ignored && tid == (int)((tgt >> 3) % kCeThreads)) {
+      const float logit = __bfloat162float(br[tgt]);
+      gr[tgt] = __float2bfloat16_rn((exp_ftz(logit - m) / s - 1.0f) * scale);
+      loss_out[row] = m + logf(s) - logit;
+    } else if (ignored && tid == 0) {
+      loss_out[row] = 0.0f;
+    }
+    tgt = next_tgt;
+    __syncthreads();  // everybody has read the row
+    if (tid == 0 && row + gridDim.x < rows) load(row + gridDim.x);
+  }
+}
+
+// valid = number of targets != ignore_index (at least 1), scale = loss_scale / valid
+__global__ void __launch_bounds__(1024)
+cross_entropy_scale_kernel(const long long* __restrict__ targets, long long rows,
+                           long long ignore_index, float loss_scale, float* __restrict__ valid,
+                           float* __restrict__ scale) {
+  __shared__ int part[32];
+  int n = 0;
+  for (long long i = threadIdx.x; i < rows; i += 1024) n += targets[i] != ignore_index;
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = n;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    n = __reduce_add_sync(0xffffffffu, part[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      const float v = (float)(n > 0 ? n : 1);
+      *valid = v;
+      *scale = loss_scale / v;
+    }
+  }
+}
+
+// loss = sum(per_row) * scale, one CTA, fixed order
+__global__ void __launch_bounds__(1024)
+cross_entropy_sum_kernel(const float* __restrict__ per_row, long long rows,
+                         const float* __restrict__ scale, float* __restrict__ loss) {
+  __shared__ float scratch[33];
+  float v = 0.0f;
+  for (long long i = threadIdx.x; i < rows; i += 1024) v += per_row[i];
+  v = block_sum(v, scratch);
+  if (threadIdx.x == 0) *loss = v * *scale;
+}
+
+// x *= bf16(s[0]) over n bf16 elements (n % 8 == 0).  The gradient that reaches a loss is almost
+// always 1: the factor is looked at on the device and the pass over x is then left away
+// (x * 1 == x for every bf16 value).  As a torch multiply by a 0-dim tensor it took 280 us at
+// 4096 x 32000 and 880 us at 8192 x 50432, longer than the cross-entropy itself; now 2 us when
+// the factor is 1.
+__global__ void __launch_bounds__(256)
+scale_inplace_kernel(bf16* __restrict__ x, long long vecs, const float* __restrict__ s) {
+  const float f = __bfloat162float(__float2bfloat16_rn(s[0]));
+  if (f == 1.0f) return;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs;
+       i += (long long)gridDim.x * blockDim.x) {
+    float v[8];
+    load8(x + i * 8, v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] *= f;
+    store8(x + i * 8, v);
   }
 }
 
@@ -714,10 +914,22 @@ sgd_momentum_kernel(float* __restrict__ param, float* __restrict__ grad, float* 
   }
 }
 
-static int grid_for(long long work, int threads) {
+// below this a row does not fill the 512 threads (4096 rows: 21.3 -> 25.5 us at 2048, 29.4 ->
+// 29.6 at 4096, 45.9 -> 37.9 at 8192, 88 -> 63 at 16384)
+constexpr int kCeMinVocab = 8192;
+// 228 KiB per SM, 1 KiB of it taken by each CTA
+constexpr int kCeMaxSmem = (228 / 2 - 1) * 1024;
+constexpr int kCeMaxSmem3 = (228 / 3 - 1) * 1024;
+
+static int sm_count() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+static int grid_for(long long work, int threads) {
+  const int sms = sm_count();
   long long g = (work + threads - 1) / threads;
   const long long cap = (long long)sms * 8;
   if (g > cap) g = cap;
@@ -878,11 +1090,55 @@ int bcom_cross_entropy(void* logits, const void* targets, void* loss_out, const 
                        int rows, int V, long long ignore_index, void* stream) {
   if (rows <= 0) return 0;
   if (V % 8) return (int)cudaErrorInvalidValue;
+  const int smem = (int)sizeof(CeShared) + 2 * V;
+  if (V >= kCeMinVocab && smem <= kCeMaxSmem && ((uintptr_t)logits & 15) == 0) {
+    const bool three = smem <= kCeMaxSmem3;
+    auto kernel = three ? cross_entropy_rows_kernel<3> : cross_entropy_rows_kernel<2>;
+    if (!tc::ensure_dynamic_smem((const void*)kernel, three ? kCeMaxSmem3 : kCeMaxSmem))
+      return (int)cudaErrorInvalidValue;
+    const int most = sm_count() * (three ? 3 : 2);
+    kernel<<<rows < most ? rows : most, kCeThreads, smem, (cudaStream_t)stream>>>(
+        (bf16*)logits, (const long long*)targets, (float*)loss_out, (const float*)grad_scale,
+        rows, V, ignore_index);
+    return (int)cudaGetLastError();
+  }
   const int grid = rows < 148 * 4 ? rows : 148 * 4;
   cross_entropy_kernel<<<grid, 512, 0, (cudaStream_t)stream>>>(
       (bf16*)logits, (const long long*)targets, (float*)loss_out, (const float*)grad_scale, rows,
       V, ignore_index);
   return (int)cudaGetLastError();
+}
+
+// valid[0] = max(1, #targets != ignore_index), scale[0] = loss_scale / valid (fp32 each)
+int bcom_cross_entropy_scale(const void* targets, long long rows, long long ignore_index,
+                             float loss_scale, void* valid, void* scale, void* stream) {
+  cross_entropy_scale_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(
+      (const long long*)targets, rows, ignore_index, loss_scale, (float*)valid, (float*)scale);
+  return (int)cudaGetLastError();
+}
+
+int bcom_cross_entropy_sum(const void* per_row, long long rows, const void* scale, void* loss,
+                           void* stream) {
+  cross_entropy_sum_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(
+      (const float*)per_row, rows, (const float*)scale, (float*)loss);
+  return (int)cudaGetLastError();
+}
+
+// x (bf16, n % 8 == 0, 16-byte aligned) *= bf16(factor[0])
+int bcom_scale_bf16(void* x, long long n, const void* factor, void* stream) {
+  if (n <= 0) return 0;
+  if ((n % 8) || ((uintptr_t)x & 15)) return (int)cudaErrorInvalidValue;
+  scale_inplace_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>(
+      (bf16*)x, n / 8, (const float*)factor);
+  return (int)cudaGetLastError();
+}
+
+// 0, or the wait that ran out in a cross-entropy launch; cleared when `clear` != 0
+int bcom_cross_entropy_status(unsigned int* out, int clear) {
+  cudaError_t err = cudaMemcpyFromSymbol(out, g_ce_status, sizeof(unsigned int));
+  const unsigned int zero = 0;
+  if (err == cudaSuccess && clear) err = cudaMemcpyToSymbol(g_ce_status, &zero, sizeof(zero));
+  return (int)err;
 }
 
 int bcom_embedding_fwd(const void* ids, const void* table, void* out, long long tokens, int H,

@@ -34,6 +34,10 @@ def _get():
             lib.bcom_swiglu_fwd.argtypes = [vp, vp, ll, ci, vp]
             lib.bcom_swiglu_bwd.argtypes = [vp, vp, vp, ll, ci, vp]
             lib.bcom_cross_entropy.argtypes = [vp, vp, vp, vp, ci, ci, ll, vp]
+            lib.bcom_cross_entropy_scale.argtypes = [vp, ll, ll, cf, vp, vp, vp]
+            lib.bcom_cross_entropy_sum.argtypes = [vp, ll, vp, vp, vp]
+            lib.bcom_scale_bf16.argtypes = [vp, ll, vp, vp]
+            lib.bcom_cross_entropy_status.argtypes = [ctypes.POINTER(ctypes.c_uint), ci]
             lib.bcom_embedding_fwd.argtypes = [vp, vp, vp, ll, ci, ci, vp]
             lib.bcom_embedding_bwd.argtypes = [vp, vp, vp, ll, ci, ci, vp]
             lib.bcom_adamw.argtypes = [vp, vp, vp, vp, vp, ll, cf, cf, cf, cf, cf, ci, cf, ci, vp]
@@ -352,6 +356,15 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
 
 
 # ----------------------------------------------------------------------------------
+def check_status(clear: bool = True) -> None:
+    """Raise if a cross-entropy kernel gave up on its bounded wait (synchronises)."""
+    out = ctypes.c_uint()
+    check(_need().bcom_cross_entropy_status(ctypes.byref(out), int(clear)),
+          "cross_entropy_status", launches=0)
+    if out.value:
+        raise NativeError("cross-entropy: a row's copy into shared memory timed out")
+
+
 class CrossEntropyFunction(torch.autograd.Function):
     """Mean token cross-entropy over non-ignored targets.  The logits buffer is consumed:
     the kernel writes d(loss)/d(logits) into it during the forward pass, so the backward
@@ -362,9 +375,9 @@ class CrossEntropyFunction(torch.autograd.Function):
         V = logits.shape[-1]
         l2 = logits.view(-1, V)
         t = targets.reshape(-1).to(torch.int64).contiguous()
-        valid = (t != ignore_index).sum().clamp_(min=1).to(torch.float32)
-        scale = (loss_scale / valid).reshape(1).contiguous()
         if not logits.is_cuda:  # the kernel's arithmetic in torch ops, for CPU ranks
+            valid = (t != ignore_index).sum().clamp_(min=1).to(torch.float32)
+            scale = (loss_scale / valid).reshape(1).contiguous()
             keep = t != ignore_index
             z = l2.float()
             lse = torch.logsumexp(z, dim=-1)
@@ -379,18 +392,31 @@ class CrossEntropyFunction(torch.autograd.Function):
             ctx.mark_non_differentiable(valid)
             return per_row.sum() * scale[0], valid
         lib = _need()
-        per_row = torch.empty(l2.shape[0], dtype=torch.float32, device=logits.device)
-        check(lib.bcom_cross_entropy(ptr(l2), ptr(t), ptr(per_row), ptr(scale), l2.shape[0], V,
-                                     int(ignore_index), stream_ptr(logits.device)),
-              "cross_entropy")
+        rows, stream = l2.shape[0], stream_ptr(logits.device)
+        per_row = torch.empty(rows, dtype=torch.float32, device=logits.device)
+        loss, valid, scale = torch.empty(3, dtype=torch.float32, device=logits.device).unbind()
+        # target count and scale, the rows, their sum: three launches
+        check(lib.bcom_cross_entropy_scale(ptr(t), rows, int(ignore_index), float(loss_scale),
+                                           ptr(valid), ptr(scale), stream), "cross_entropy_scale")
+        check(lib.bcom_cross_entropy(ptr(l2), ptr(t), ptr(per_row), ptr(scale), rows, V,
+                                     int(ignore_index), stream), "cross_entropy")
+        check(lib.bcom_cross_entropy_sum(ptr(per_row), rows, ptr(scale), ptr(loss), stream),
+              "cross_entropy_sum")
         ctx.save_for_backward(logits)
         ctx.mark_non_differentiable(valid)
-        return per_row.sum() * scale[0], valid
+        return loss, valid
 
     @staticmethod
     def backward(ctx, dloss, _dvalid):
         (dlogits,) = ctx.saved_tensors
         # the buffer already holds d(loss)/d(logits); scale it by the incoming gradient
+        if (dlogits.is_cuda and dlogits.is_contiguous() and dlogits.data_ptr() % 16 == 0
+                and dloss.dtype == torch.float32 and not torch.is_grad_enabled()):
+            check(_need().bcom_scale_bf16(ptr(dlogits), dlogits.numel(), ptr(dloss),
+                                          stream_ptr(dlogits.device)), "scale_bf16")
+            # an in-place change like mul_: a second backward pass over the buffer is refused
+            torch.autograd.graph.increment_version(dlogits)
+            return dlogits, None, None, None
         return dlogits.mul_(dloss.to(dlogits.dtype)), None, None, None
 
 

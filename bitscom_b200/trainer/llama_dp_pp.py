@@ -335,11 +335,13 @@ class LlamaTrainer:
         a checkpoint replaces the last good file."""
         from ..ops import attention as A
         from ..ops import gemm as G
+        from ..ops import nn as K
 
         if self.device.type != "cuda":
             return
         if G.available():
             G.check_status()
+            K.check_status()
         if A.available():
             A.check_status()
         if self.syncs:

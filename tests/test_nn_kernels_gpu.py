@@ -160,6 +160,29 @@ def test_cross_entropy_loss_and_grad(rows, V):
     assert torch.allclose(work.grad.float(), ref_in.grad, rtol=5e-2, atol=2e-4)
 
 
+@pytest.mark.parametrize("rows,V", [(3, 8184), (5, 8192), (700, 38272), (450, 38400), (300, 50432),
+                                    (299, 57728), (7, 57856)])
+@pytest.mark.parametrize("upstream", [1.0, -2.5])
+def test_cross_entropy_vocabulary_rows(rows, V, upstream):
+    """Around the sizes where the kernel changes (8192; 38.3 k and 57.8 k, where three and two
+    rows fit an SM), with masked words, a fully masked stretch and a gradient that is not 1.
+    Bounds: bf16 results of fp32 arithmetic round to 2^-9 relative, twice when scaled."""
+    logits = _bf(rows, V, seed=V, scale=2.0)
+    logits[:, 64:4096] = float("-inf")
+    logits[0, 4100] = torch.finfo(torch.bfloat16).min
+    targets = torch.randint(4200, V, (rows,), device="cuda")
+    targets[0], targets[1], targets[2] = V - 1, 0, V - 8
+    ref_in = logits.float().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(ref_in, targets, ignore_index=0)
+    ref.backward(torch.tensor(upstream, device="cuda"))
+    work = logits.clone().requires_grad_()
+    loss = K.cross_entropy(work * 1.0, targets, ignore_index=0)
+    loss.backward(torch.tensor(upstream, device="cuda"))
+    K.check_status()
+    assert abs(loss.item() - ref.item()) < 1e-5 * abs(ref.item())
+    assert torch.allclose(work.grad.float(), ref_in.grad, rtol=2 ** -7, atol=1e-9)
+
+
 def test_embedding_fwd_bwd():
     V, H, T = 1000, 256, 300
     table = _bf(V, H, seed=9).requires_grad_()
