@@ -365,7 +365,7 @@ def main(argv=None):
     ap.add_argument("--n", type=int, default=4096)
     ap.add_argument("--k", type=int, default=4096)
     ap.add_argument("--wgrad", action="store_true")
-    ap.add_argument("--gemm-variant", default="1cta", choices=["1cta", "2cta"])
+    ap.add_argument("--gemm-variant", default="auto", choices=["auto", "1cta", "2cta"])
     ap.add_argument("--iters", type=int, default=5)
     ap.add_argument("--warmup", type=int, default=3)
     args = ap.parse_args(argv)

@@ -159,46 +159,51 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = tc::make_idesc_bf16(BM, BN, A_MN, B_MN);
-      int stage = 0;
-      uint32_t phase = 0;
-      int iter = 0;
-      for (int t = blockIdx.x; t < total_tiles && !sh->abort; t += gridDim.x, ++iter) {
-        const int buf = iter & 1;
-        const uint32_t acc_phase = (uint32_t)(iter >> 1) & 1u;
-        if (!tc::mbar_wait(&sh->acc_empty[buf], acc_phase ^ 1u, kWaitBudgetNs)) {
-          fail(sh, kAccumTimeout);
+    // The whole warp walks the loop and one elected lane issues: with `if (lane == 0)` around
+    // the loop every descriptor and address is a per-thread value that has to be moved into the
+    // uniform registers the MMA takes, and that issue work, not the tensor pipe, set the pace
+    // (share of the peak at the sampled clock, 8192^3: 0.75 -> 0.77 here, where the operands'
+    // way through shared memory is next, 0.73 -> 0.88 in the CTA-pair kernel; cuBLAS 0.87).
+    constexpr uint32_t idesc = tc::make_idesc_bf16(BM, BN, A_MN, B_MN);
+    constexpr uint32_t hi = tc::desc_hi(1024);
+    constexpr uint32_t a_step = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+    constexpr uint32_t b_step = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+    const uint32_t a_lo0 = tc::desc_lo(tc::smem_u32(smem), A_MN ? CHUNK_BYTES : 16);
+    const uint32_t b_lo0 = tc::desc_lo(tc::smem_u32(smem) + A_BYTES, B_MN ? CHUNK_BYTES : 16);
+    int stage = 0;
+    uint32_t phase = 0;
+    int iter = 0;
+    for (int t = blockIdx.x; t < total_tiles && !sh->abort; t += gridDim.x, ++iter) {
+      const int buf = iter & 1;
+      const uint32_t acc_phase = (uint32_t)(iter >> 1) & 1u;
+      if (!tc::mbar_wait_warp(&sh->acc_empty[buf], acc_phase ^ 1u, kWaitBudgetNs)) {
+        if (lane == 0) fail(sh, kAccumTimeout);
+        break;
+      }
+      tc::tc_fence_after_sync();
+      const uint32_t d_tmem = tmem_base + (uint32_t)buf * BN;
+      bool ok = true;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!tc::mbar_wait_warp(&sh->full[stage], phase, kWaitBudgetNs)) {
+          if (lane == 0) fail(sh, kMmaTimeout);
+          ok = false;
           break;
         }
         tc::tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + (uint32_t)buf * BN;
-        bool ok = true;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!tc::mbar_wait(&sh->full[stage], phase, kWaitBudgetNs)) {
-            fail(sh, kMmaTimeout);
-            ok = false;
-            break;
-          }
-          tc::tc_fence_after_sync();
-          const uint32_t a_addr = tc::smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_BYTES;
+        const uint32_t a_lo = a_lo0 + stage * (STAGE_BYTES >> 4);
+        const uint32_t b_lo = b_lo0 + stage * (STAGE_BYTES >> 4);
+        if (tc::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t da = A_MN
-                ? tc::make_smem_desc_sw128(a_addr + k * (UMMA_K * 128), CHUNK_BYTES, 1024)
-                : tc::make_smem_desc_sw128(a_addr + k * (UMMA_K * 2), 16, 1024);
-            const uint64_t db = B_MN
-                ? tc::make_smem_desc_sw128(b_addr + k * (UMMA_K * 128), CHUNK_BYTES, 1024)
-                : tc::make_smem_desc_sw128(b_addr + k * (UMMA_K * 2), 16, 1024);
-            tc::umma_bf16(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            tc::umma_bf16_lo<1>(d_tmem, a_lo + k * a_step, hi, b_lo + k * b_step, hi, idesc,
+                                (kb | k) != 0 ? 1u : 0u);
           tc::umma_commit(&sh->empty[stage]);  // stage reusable once these MMAs are done
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          if (kb == num_kb - 1) tc::umma_commit(&sh->acc_full[buf]);
         }
-        if (!ok) break;
-        tc::umma_commit(&sh->acc_full[buf]);
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
+      if (!ok) break;
     }
   } else {
     // ------------------------------ epilogue -----------------------------------

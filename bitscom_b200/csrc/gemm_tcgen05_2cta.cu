@@ -130,6 +130,14 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
   return true;
 }
 
+// the same by a whole warp, with a uniform verdict
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity,
+                                                       unsigned long long budget_ns) {
+  if (__all_sync(0xffffffffu, mbar_try_wait_cluster(bar, parity))) return true;
+  const bool ok = mbar_wait_cluster(bar, parity, budget_ns);
+  return __all_sync(0xffffffffu, ok);
+}
+
 // One warp of EACH CTA of the pair executes these.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_out, uint32_t columns) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -143,31 +151,14 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t base, uint32_t column
                : "memory");
 }
 
-// D[tmem of both CTAs] (+)= A[smem of both] * B[smem of both]; issued by ONE thread of the leader.
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                               uint32_t idesc, uint32_t accumulate) {
+// The barrier at this offset in both CTAs of the pair receives one arrival once all tcgen05
+// operations issued so far by this thread have completed.
+__device__ __forceinline__ void umma_commit_both(uint64_t* bar) {
   asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
+      " [%0], %1;" ::"r"(tc::smem_u32(bar)),
+      "h"((uint16_t)3)
       : "memory");
-}
-// The barrier at shared::cluster address `bar` (this CTA's or the peer's) receives one arrival
-// once all tcgen05 operations issued so far by this thread have completed.
-__device__ __forceinline__ void umma_commit_to(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   bar)
-               : "memory");
-}
-// Both CTAs of the pair: the barrier at this offset here, and the one at the same offset in the
-// peer (`peer_bar` = map_to_cta(bar, 1)).
-__device__ __forceinline__ void umma_commit_both(uint64_t* bar, uint32_t peer_bar) {
-  umma_commit_to(tc::smem_u32(bar));
-  umma_commit_to(peer_bar);
 }
 // 2-D tiled load of the CTA-pair form: the data lands in THIS CTA's shared memory, the bytes
 // are counted on the barrier at shared::cluster address `bar`, which may be the peer's.
@@ -283,21 +274,27 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
       // ------------------------------ MMA issuer (leader) ----------------------
+      // The whole warp walks the loop, one elected lane issues (see gemm_tcgen05.cu).
       constexpr uint32_t idesc = tc::make_idesc_bf16(BM, BN, A_MN, B_MN);
+      constexpr uint32_t hi = tc::desc_hi(1024);
+      constexpr uint32_t a_step = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+      constexpr uint32_t b_step = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+      const uint32_t a_lo0 = tc::desc_lo(tc::smem_u32(smem), A_MN ? CHUNK_BYTES : 16);
+      const uint32_t b_lo0 = tc::desc_lo(tc::smem_u32(smem) + A_BYTES, B_MN ? CHUNK_BYTES : 16);
       int stage = 0;
       uint32_t phase = 0;
       int iter = 0;
       unsigned long long* const prof = g_profile;
-      long long t_full = 0, t_acc = 0, n_kb = 0;
+      long long t_full = 0, t_acc = 0, n_kb = 0, c0 = 0;
       const long long t_begin = prof ? clock64() : 0;
       for (int t = pair; t < total_tiles && !sh->abort; t += num_pairs, ++iter) {
         const int buf = iter & 1;
         const uint32_t acc_phase = (uint32_t)(iter >> 1) & 1u;
-        long long c0 = prof ? clock64() : 0;
-        if (!mbar_wait_cluster(&sh->acc_empty[buf], acc_phase ^ 1u, kWaitBudgetNs)) {
-          fail(sh, kAccumTimeout);
+        if (prof) c0 = clock64();
+        if (!mbar_wait_cluster_warp(&sh->acc_empty[buf], acc_phase ^ 1u, kWaitBudgetNs)) {
+          if (lane == 0) fail(sh, kAccumTimeout);
           break;
         }
         if (prof) t_acc += clock64() - c0;
@@ -307,33 +304,29 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         for (int kb = 0; kb < num_kb; ++kb) {
           if (prof) c0 = clock64();
           // the odd CTA's bytes arrive from the other SM: cluster-scope acquire
-          if (!mbar_wait_cluster(&sh->full[stage], phase, kWaitBudgetNs)) {
-            fail(sh, kMmaTimeout);
+          if (!mbar_wait_cluster_warp(&sh->full[stage], phase, kWaitBudgetNs)) {
+            if (lane == 0) fail(sh, kMmaTimeout);
             ok = false;
             break;
           }
           if (prof) { t_full += clock64() - c0; ++n_kb; }
           tc::tc_fence_after_sync();
-          const uint32_t a_addr = tc::smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_BYTES;
+          const uint32_t a_lo = a_lo0 + stage * (STAGE_BYTES >> 4);
+          const uint32_t b_lo = b_lo0 + stage * (STAGE_BYTES >> 4);
+          if (tc::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t da = A_MN
-                ? tc::make_smem_desc_sw128(a_addr + k * (UMMA_K * 128), CHUNK_BYTES, 1024)
-                : tc::make_smem_desc_sw128(a_addr + k * (UMMA_K * 2), 16, 1024);
-            const uint64_t db = B_MN
-                ? tc::make_smem_desc_sw128(b_addr + k * (UMMA_K * 128), CHUNK_BYTES, 1024)
-                : tc::make_smem_desc_sw128(b_addr + k * (UMMA_K * 2), 16, 1024);
-            umma_bf16_pair(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              tc::umma_bf16_lo<2>(d_tmem, a_lo + k * a_step, hi, b_lo + k * b_step, hi, idesc,
+                                  (kb | k) != 0 ? 1u : 0u);
+            umma_commit_both(&sh->empty[stage]);  // both CTAs may refill the stage
+            if (kb == num_kb - 1) umma_commit_both(&sh->acc_full[buf]);
           }
-          // both CTAs may refill the stage
-          umma_commit_both(&sh->empty[stage], map_to_cta(&sh->empty[stage], 1));
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        umma_commit_both(&sh->acc_full[buf], map_to_cta(&sh->acc_full[buf], 1));
       }
-      if (prof) {
+      if (prof && lane == 0) {
         prof[4 * pair + 0] = (unsigned long long)t_full;
         prof[4 * pair + 1] = (unsigned long long)t_acc;
         prof[4 * pair + 2] = (unsigned long long)(clock64() - t_begin);

@@ -90,6 +90,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return true;
 }
 
+// The same wait by a whole warp: the verdict is uniform, so the warp stays converged and what
+// follows (descriptors, loop state) can live in uniform registers.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
+                                               unsigned long long budget_ns) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const bool ok = mbar_wait(bar, parity, budget_ns);
+  return __all_sync(0xffffffffu, ok);
+}
+
 // ---------------------------------------------------------------------------
 // TMA: 2-D tiled load, global -> shared, completion on an mbarrier
 // (coordinate 0 is the contiguous dimension; c0 * elem_size must be a multiple of 16)
@@ -241,6 +250,50 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint
       :
       : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+
+// The same instruction with descriptors given as two 32-bit words.  A tile's descriptors differ
+// only in the low word (start address), by a constant per k-step, so an issuer that keeps the
+// low words spends one add per operand instead of assembling 64 bits each time.
+template <int CTA_GROUP>
+__device__ __forceinline__ void umma_bf16_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi,
+                                             uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                             uint32_t accumulate) {
+  if constexpr (CTA_GROUP == 1) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 da, {%1, %2};\n\t"
+        "mov.b64 db, {%3, %4};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t"
+        "}\n"
+        :
+        : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 da, {%1, %2};\n\t"
+        "mov.b64 db, {%3, %4};\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t"
+        "}\n"
+        :
+        : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+  }
+}
+// low / high word of make_smem_desc_sw128; the low word of a tile `bytes` further on is
+// desc_lo + (bytes >> 4) (shared-memory addresses stay below 2^18)
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
+  return (smem_addr >> 4) | ((lbo_bytes >> 4) << 16);
+}
+__host__ __device__ constexpr uint32_t desc_hi(uint32_t sbo_bytes) {
+  return (sbo_bytes >> 4) | (1u << 14) | (2u << 29);
 }
 
 // mbarrier arrives once all tcgen05 ops issued so far by this thread have completed

@@ -17,8 +17,8 @@ from ._native import NativeError, check, ptr, stream_ptr
 
 _lib = None
 _lib2 = None      # the CTA-pair kernel's library, loaded when that variant is first selected
-_variant = None   # "1cta" | "2cta"; None until the first call reads BITSCOM_GEMM
-_VARIANTS = ("1cta", "2cta")
+_variant = None   # one of _VARIANTS; None until the first call reads BITSCOM_GEMM
+_VARIANTS = ("auto", "1cta", "2cta")
 
 
 def _get():
@@ -68,17 +68,26 @@ def available() -> bool:
 
 
 def variant() -> str:
-    """The kernel that ``gemm`` launches: "1cta" (default) or "2cta" (CTA pairs, 256x256 tiles,
-    ``tcgen05.mma.cta_group::2``).  Initialised from ``BITSCOM_GEMM``."""
+    """The kernel that ``gemm`` launches: "1cta", "2cta" (CTA pairs, 256x256 tiles,
+    ``tcgen05.mma.cta_group::2``) or "auto" (default: by shape, see ``_use_pair``).  Initialised
+    from ``BITSCOM_GEMM``."""
     global _variant
     if _variant is None:
-        want = os.environ.get("BITSCOM_GEMM", "1cta").strip().lower()
-        _variant = "1cta"
-        if want == "2cta":
-            set_variant("2cta")
-        elif want != "1cta":
+        want = os.environ.get("BITSCOM_GEMM", "auto").strip().lower()
+        if want not in _VARIANTS:
             raise ValueError(f"BITSCOM_GEMM={want!r}: expected one of {_VARIANTS}")
+        _variant = "auto"
+        if want != "auto":
+            set_variant(want)
     return _variant
+
+
+def _use_pair(M: int, N: int) -> bool:
+    """More than one wave of 128x256 tiles: CTA pairs, which read half as much of B per SM and
+    keep the tensor pipe busier (4096 x 22016 x 4096: 548 -> 508 us, its weight gradient 661 ->
+    601 us).  Up to one wave the pairs' 256-row tiles leave more of the chip idle than they
+    save (1024 x 4096 x 4096: 26.7 -> 28.7 us)."""
+    return -(-M // 128) * -(-N // 256) > 148 and _get2() is not None
 
 
 def set_variant(name: str) -> str:
@@ -87,7 +96,7 @@ def set_variant(name: str) -> str:
     global _variant
     if name not in _VARIANTS:
         raise ValueError(f"unknown GEMM variant {name!r}")
-    old = _variant or "1cta"
+    old = _variant or "auto"
     if name == "2cta" and _get2() is None:
         raise NativeError("the CTA-pair GEMM needs the bcom_gemm2 library and a GPU")
     _variant = name
@@ -197,7 +206,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False,
     if residual is not None and (residual.shape != (M, N) or residual.stride(1) != 1
                                  or residual.dtype != torch.bfloat16):
         raise ValueError("bad residual tensor")
-    launch = lib.bcom_gemm_bf16_ex if variant() == "1cta" else _get2().bcom_gemm2_bf16_ex
+    kind = variant()
+    pair = max_ctas != 1 and _use_pair(M, N) if kind == "auto" else kind == "2cta"
+    launch = _get2().bcom_gemm2_bf16_ex if pair else lib.bcom_gemm_bf16_ex
     with _native.on_device(a.device):
         check(launch(
             ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K, a.stride(0), b.stride(0),
