@@ -49,7 +49,7 @@ constexpr int kThreads = 192;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr int GROUP_M = 8;
 constexpr unsigned long long kWaitBudgetNs = 2000000000ull;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*alignment slack*/ + 256;
 
 enum Status : unsigned int {
   kOk = 0, kProducerTimeout = 1, kMmaTimeout = 2, kEpilogueTimeout = 3, kAccumTimeout = 4
@@ -91,11 +91,12 @@ __device__ __forceinline__ WorkItem work_item(const Params& p, int w) {
 template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const Params p) {
+                 const __grid_constant__ CUtensorMap tmC, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  Shared* sh = reinterpret_cast<Shared*>(smem + STAGES * STAGE_BYTES);
+  uint8_t* epi = smem + STAGES * STAGE_BYTES;
+  Shared* sh = reinterpret_cast<Shared*>(epi + EPI_BYTES);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -218,15 +219,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         break;
       }
       tc::tc_fence_after_sync();
-      const int row = wi.m0 + quarter * 32 + lane;
-      const int n0 = wi.n0;
       const uint32_t taddr = tmem_base + (uint32_t)buf * BN + ((uint32_t)(quarter * 32) << 16);
-      store_accumulator_rows<BN, OUT_F32, ACCUM>(taddr, p.C, p.ldc, row, n0, p.M, p.N, p.R,
-                                                 p.ldr);
+      write_accumulator<BN, OUT_F32, ACCUM>(taddr, &tmC, epi + quarter * EPI_WARP_BYTES, p.C, p.ldc,
+                                            wi.m0 + quarter * 32, wi.n0, p.M, p.N, p.R, p.ldr,
+                                            lane);
       tc::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&sh->acc_empty[buf]);
     }
+    if (lane == 0) tc::bulk_wait_group0();  // C is written before the CTA leaves
   }
 
   // ------------------------------ teardown -------------------------------------
@@ -247,7 +248,7 @@ static int make_map(CUtensorMap* map, const void* ptr, long long rows, long long
   return tc::cached_tensor_map_2d(map, ptr, 2, rows, cols, ld, box_cols, box_rows);
 }
 
-typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const Params);
+typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const Params);
 
 template <bool A_MN, bool B_MN>
 static Kernel pick_out(bool out_f32, bool accum) {
@@ -286,7 +287,7 @@ int bcom_gemm_bf16_ex(const void* A, const void* B, void* C, const void* residua
   if (((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15)) return 1002;
   if (residual && (out_fp32 || accumulate || (ldr % 8) || ((uintptr_t)residual & 15))) return 1001;
   (void)cudaGetLastError();  // do not inherit an error left behind by an earlier call
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC;
   // the tensor-map encoder is a driver call: make sure this thread (it may be an autograd
   // worker) has the device's primary context bound
   tc::bind_context_once();
@@ -312,9 +313,10 @@ int bcom_gemm_bf16_ex(const void* A, const void* B, void* C, const void* residua
   if (b_mn_major ? make_map(&tmB, B, K, N, ldb, 64, BK)
                  : make_map(&tmB, B, N, K, ldb, BK, BN))
     return 1004;
+  if (make_c_map(&tmC, C, M, N, ldc, out_fp32 != 0)) return 1008;
   Kernel kernel = pick(a_mn_major != 0, b_mn_major != 0, out_fp32 != 0, accumulate != 0);
   if (!tc::ensure_dynamic_smem((const void*)kernel, SMEM_BYTES)) return 1005;
-  kernel<<<grid, kThreads, SMEM_BYTES, (cudaStream_t)stream>>>(tmA, tmB, p);
+  kernel<<<grid, kThreads, SMEM_BYTES, (cudaStream_t)stream>>>(tmA, tmB, tmC, p);
   return (int)cudaGetLastError();
 }
 

@@ -50,7 +50,7 @@ constexpr int kThreads = 192;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr int GROUP_M = 8;
 constexpr unsigned long long kWaitBudgetNs = 2000000000ull;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + gemm::EPI_BYTES + 1024 /*alignment slack*/ + 256;
 
 enum Status : unsigned int {
   kOk = 0, kProducerTimeout = 1, kMmaTimeout = 2, kEpilogueTimeout = 3, kAccumTimeout = 4
@@ -187,11 +187,13 @@ __device__ __forceinline__ void tile_coords(const Params& p, int t, int* tm, int
 template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
-                      const __grid_constant__ CUtensorMap tmB, const Params p) {
+                      const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ CUtensorMap tmC, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  Shared* sh = reinterpret_cast<Shared*>(smem + STAGES * STAGE_BYTES);
+  uint8_t* epi = smem + STAGES * STAGE_BYTES;
+  Shared* sh = reinterpret_cast<Shared*>(epi + gemm::EPI_BYTES);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -347,11 +349,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         break;
       }
       tc::tc_fence_after_sync();
-      const int row = tm * BM + (int)rank * BM_CTA + quarter * 32 + lane;
-      const int n0 = tn * BN;
       const uint32_t taddr = tmem_base + (uint32_t)buf * BN + ((uint32_t)(quarter * 32) << 16);
-      gemm::store_accumulator_rows<BN, OUT_F32, ACCUM>(taddr, p.C, p.ldc, row, n0, p.M, p.N, p.R,
-                                                       p.ldr);
+      gemm::write_accumulator<BN, OUT_F32, ACCUM>(
+          taddr, &tmC, epi + quarter * gemm::EPI_WARP_BYTES, p.C, p.ldc,
+          tm * BM + (int)rank * BM_CTA + quarter * 32, tn * BN, p.M, p.N, p.R, p.ldr, lane);
       tc::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
@@ -359,6 +360,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
         else mbar_arrive_cluster(map_to_cta(&sh->acc_empty[buf], 0));
       }
     }
+    if (lane == 0) tc::bulk_wait_group0();  // C is written before the CTA leaves
   }
 
   // ------------------------------ teardown -------------------------------------
@@ -382,7 +384,7 @@ static int make_map(CUtensorMap* map, const void* ptr, long long rows, long long
   return tc::cached_tensor_map_2d(map, ptr, 2, rows, cols, ld, box_cols, box_rows);
 }
 
-typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const Params);
+typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const Params);
 
 template <bool A_MN, bool B_MN>
 static Kernel pick_out(bool out_f32, bool accum) {
@@ -443,12 +445,13 @@ int bcom_gemm2_bf16_ex(const void* A, const void* B, void* C, const void* residu
   if (((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15)) return 1002;
   if (residual && (out_fp32 || accumulate || (ldr % 8) || ((uintptr_t)residual & 15))) return 1001;
   (void)cudaGetLastError();
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC;
   tc::bind_context_once();
   if (a_mn_major ? make_map(&tmA, A, K, M, lda, 64, BK) : make_map(&tmA, A, M, K, lda, BK, BM_CTA))
     return 1003;
   if (b_mn_major ? make_map(&tmB, B, K, N, ldb, 64, BK) : make_map(&tmB, B, N, K, ldb, BK, BN_CTA))
     return 1004;
+  if (gemm::make_c_map(&tmC, C, M, N, ldc, out_fp32 != 0)) return 1008;
   Kernel kernel = pick(a_mn_major != 0, b_mn_major != 0, out_fp32 != 0, accumulate != 0);
   if (!tc::ensure_dynamic_smem((const void*)kernel, SMEM_BYTES)) return 1005;
   Params p;
@@ -468,7 +471,7 @@ int bcom_gemm2_bf16_ex(const void* A, const void* B, void* C, const void* residu
   if (pairs > tiles) pairs = tiles;
   if (max_ctas >= 2 && pairs > max_ctas / 2) pairs = max_ctas / 2;
   if (pairs < 1) pairs = 1;
-  kernel<<<2 * pairs, kThreads, SMEM_BYTES, (cudaStream_t)stream>>>(tmA, tmB, p);
+  kernel<<<2 * pairs, kThreads, SMEM_BYTES, (cudaStream_t)stream>>>(tmA, tmB, tmC, p);
   return (int)cudaGetLastError();
 }
 

@@ -140,12 +140,25 @@ __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const 
       : "l"(map), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
       : "memory");
 }
+// 2-D tiled store, shared -> global; parts of the box outside the tensor are not written
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int c0,
+                                             int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+      :
+      : "l"(map), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
+      : "memory");
+}
 __device__ __forceinline__ void bulk_commit_group() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 // all committed groups of this thread have finished READING their shared-memory source
 __device__ __forceinline__ void bulk_wait_group_read0() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+// all but the newest one have
+__device__ __forceinline__ void bulk_wait_group_read1() {
+  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
 }
 // ... have completed entirely (their global writes are performed)
 __device__ __forceinline__ void bulk_wait_group0() {

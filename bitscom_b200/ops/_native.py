@@ -71,6 +71,7 @@ _ARG_ERRORS = {
     1002: "an operand is not 16-byte aligned",
     1003: "the tensor map of A could not be encoded",
     1004: "the tensor map of B could not be encoded",
+    1008: "the tensor map of C could not be encoded",
     1005: "the kernel's shared-memory attribute could not be set",
 }
 
