@@ -31,4 +31,9 @@ __host__ __device__ inline WorkItem work_item(int tiles_m, int tiles_n, int w) {
   return WorkItem{tm * BM, tn * BN};
 }
 
+// first k-block of part `split` when `num_kb` blocks are shared out among `splits` parts
+__host__ __device__ inline int split_begin(int num_kb, int splits, int split) {
+  return (int)((long long)num_kb * split / splits);
+}
+
 }  // namespace gemm_sched

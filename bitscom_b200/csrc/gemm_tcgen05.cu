@@ -37,19 +37,23 @@
 namespace gemm {
 
 constexpr int BM = 128;
-constexpr int BN = 256;
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int STAGES = 4;
 constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
-constexpr int B_BYTES = BN * BK * 2;  // 32 KiB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int CHUNK_BYTES = 64 * BK * 2;  // one MN-major box: 64 mn x 64 k
 constexpr int kThreads = 192;
-constexpr uint32_t TMEM_COLS = 512;
+constexpr int MAX_STAGES = 6;
+// Output tiles are 128 x 256, or 128 x 128 where that many columns leave SMs without a tile.
+template <int BN> struct Tile {
+  static constexpr int STAGES = BN == 256 ? 4 : 6;
+  static constexpr int B_BYTES = BN * BK * 2;             // 32 or 16 KiB
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;   // 192 KiB of ring in both
+  static constexpr uint32_t TMEM_COLS = 2 * BN;
+  static constexpr int SMEM_BYTES =
+      STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*alignment slack*/ + 256;
+};
 constexpr int GROUP_M = 8;
 constexpr unsigned long long kWaitBudgetNs = 2000000000ull;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*alignment slack*/ + 256;
 
 enum Status : unsigned int {
   kOk = 0, kProducerTimeout = 1, kMmaTimeout = 2, kEpilogueTimeout = 3, kAccumTimeout = 4
@@ -63,11 +67,14 @@ struct Params {
   long long ldc, ldr;
   int M, N, K;
   int tiles_m, tiles_n;
+  // K shared out among this many work items per tile; item s of a tile writes its fp32 partial
+  // tile to rows [s * split_rows, ...) of C, which is then the workspace of the call.
+  int splits, split_rows;
 };
 
 struct Shared {
-  uint64_t full[STAGES];
-  uint64_t empty[STAGES];
+  uint64_t full[MAX_STAGES];
+  uint64_t empty[MAX_STAGES];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem_base;
@@ -82,16 +89,27 @@ __device__ __forceinline__ void fail(Shared* sh, unsigned int code) {
   }
 }
 
-// One unit of work of a CTA: rows [m0, m0 + BM), columns [n0, n0 + BN) of C.
-using gemm_sched::WorkItem;
+// One unit of work of a CTA: k-blocks [kb0, kb1) of rows [m0, m0 + BM), columns [n0, n0 + BN).
+struct WorkItem {
+  int m0, n0, kb0, kb1, split;
+};
+template <int BN>
 __device__ __forceinline__ WorkItem work_item(const Params& p, int w) {
-  return gemm_sched::work_item<BM, BN, GROUP_M>(p.tiles_m, p.tiles_n, w);
+  const int tiles = p.tiles_m * p.tiles_n;
+  const int num_kb = (p.K + BK - 1) / BK;
+  const int split = p.splits == 1 ? 0 : w / tiles;
+  const gemm_sched::WorkItem t =
+      gemm_sched::work_item<BM, BN, GROUP_M>(p.tiles_m, p.tiles_n, w - split * tiles);
+  return WorkItem{t.m0, t.n0, gemm_sched::split_begin(num_kb, p.splits, split),
+                  gemm_sched::split_begin(num_kb, p.splits, split + 1), split};
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
+template <int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const Params p) {
+  constexpr int STAGES = Tile<BN>::STAGES, STAGE_BYTES = Tile<BN>::STAGE_BYTES;
+  constexpr uint32_t TMEM_COLS = Tile<BN>::TMEM_COLS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -100,8 +118,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int num_kb = (p.K + BK - 1) / BK;
-  const int total_tiles = p.tiles_m * p.tiles_n;
+  const int total_tiles = p.tiles_m * p.tiles_n * p.splits;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -129,9 +146,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int stage = 0;
       uint32_t phase = 0;
       for (int t = blockIdx.x; t < total_tiles && !sh->abort; t += gridDim.x) {
-        const WorkItem wi = work_item(p, t);
+        const WorkItem wi = work_item<BN>(p, t);
         const int m0 = wi.m0, n0 = wi.n0;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = wi.kb0; kb < wi.kb1; ++kb) {
           if (!tc::mbar_wait(&sh->empty[stage], phase ^ 1u, kWaitBudgetNs)) {
             fail(sh, kProducerTimeout);
             break;
@@ -183,8 +200,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       tc::tc_fence_after_sync();
       const uint32_t d_tmem = tmem_base + (uint32_t)buf * BN;
+      const WorkItem wi = work_item<BN>(p, t);
       bool ok = true;
-      for (int kb = 0; kb < num_kb; ++kb) {
+      for (int kb = wi.kb0; kb < wi.kb1; ++kb) {
         if (!tc::mbar_wait_warp(&sh->full[stage], phase, kWaitBudgetNs)) {
           if (lane == 0) fail(sh, kMmaTimeout);
           ok = false;
@@ -197,9 +215,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
             tc::umma_bf16_lo<1>(d_tmem, a_lo + k * a_step, hi, b_lo + k * b_step, hi, idesc,
-                                (kb | k) != 0 ? 1u : 0u);
+                                kb != wi.kb0 || k != 0 ? 1u : 0u);
           tc::umma_commit(&sh->empty[stage]);  // stage reusable once these MMAs are done
-          if (kb == num_kb - 1) tc::umma_commit(&sh->acc_full[buf]);
+          if (kb == wi.kb1 - 1) tc::umma_commit(&sh->acc_full[buf]);
         }
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -211,7 +229,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int quarter = warp & 3;  // TMEM lanes this warp may read: 32*quarter ..
     int iter = 0;
     for (int t = blockIdx.x; t < total_tiles && !sh->abort; t += gridDim.x, ++iter) {
-      const WorkItem wi = work_item(p, t);
+      const WorkItem wi = work_item<BN>(p, t);
       const int buf = iter & 1;
       const uint32_t acc_phase = (uint32_t)(iter >> 1) & 1u;
       if (!tc::mbar_wait(&sh->acc_full[buf], acc_phase, kWaitBudgetNs)) {
@@ -220,9 +238,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       tc::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (uint32_t)buf * BN + ((uint32_t)(quarter * 32) << 16);
-      write_accumulator<BN, OUT_F32, ACCUM>(taddr, &tmC, epi + quarter * EPI_WARP_BYTES, p.C, p.ldc,
-                                            wi.m0 + quarter * 32, wi.n0, p.M, p.N, p.R, p.ldr,
-                                            lane);
+      const int row0 = wi.m0 + quarter * 32;
+      if (p.splits == 1)
+        write_accumulator<BN, OUT_F32, ACCUM>(taddr, &tmC, epi + quarter * EPI_WARP_BYTES, p.C,
+                                              p.ldc, row0, wi.n0, p.M, p.N, p.R, p.ldr, lane);
+      else if constexpr (OUT_F32 && !ACCUM)
+        write_accumulator<BN, true, false>(taddr, &tmC, epi + quarter * EPI_WARP_BYTES, p.C, p.ldc,
+                                           wi.split * p.split_rows + row0, wi.n0,
+                                           p.splits * p.split_rows, p.N, nullptr, 0, lane);
       tc::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&sh->acc_empty[buf]);
@@ -248,20 +271,120 @@ static int make_map(CUtensorMap* map, const void* ptr, long long rows, long long
   return tc::cached_tensor_map_2d(map, ptr, 2, rows, cols, ld, box_cols, box_rows);
 }
 
-typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const Params);
-
-template <bool A_MN, bool B_MN>
-static Kernel pick_out(bool out_f32, bool accum) {
-  if (out_f32) return accum ? gemm_bf16_kernel<A_MN, B_MN, true, true>
-                            : gemm_bf16_kernel<A_MN, B_MN, true, false>;
-  return accum ? gemm_bf16_kernel<A_MN, B_MN, false, true>
-               : gemm_bf16_kernel<A_MN, B_MN, false, false>;
+static int sm_count() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
 }
 
+typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const Params);
+
+template <int BN, bool A_MN, bool B_MN>
+static Kernel pick_out(bool out_f32, bool accum) {
+  if (out_f32) return accum ? gemm_bf16_kernel<BN, A_MN, B_MN, true, true>
+                            : gemm_bf16_kernel<BN, A_MN, B_MN, true, false>;
+  return accum ? gemm_bf16_kernel<BN, A_MN, B_MN, false, true>
+               : gemm_bf16_kernel<BN, A_MN, B_MN, false, false>;
+}
+
+template <int BN>
 static Kernel pick(bool a_mn, bool b_mn, bool out_f32, bool accum) {
-  if (a_mn) return b_mn ? pick_out<true, true>(out_f32, accum)
-                        : pick_out<true, false>(out_f32, accum);
-  return b_mn ? pick_out<false, true>(out_f32, accum) : pick_out<false, false>(out_f32, accum);
+  if (a_mn) return b_mn ? pick_out<BN, true, true>(out_f32, accum)
+                        : pick_out<BN, true, false>(out_f32, accum);
+  return b_mn ? pick_out<BN, false, true>(out_f32, accum)
+              : pick_out<BN, false, false>(out_f32, accum);
+}
+
+// C (bf16 or fp32) = sum over splits of the partial tiles, in ascending order (+ residual or + C).
+// Reads what the product kernel has just written (it is still in the L2).
+template <bool OUT_F32, bool ACCUM>
+__global__ void __launch_bounds__(256)
+split_sum_kernel(const float* __restrict__ ws, int splits, long long split_stride, void* C,
+                 const __nv_bfloat16* __restrict__ R, long long ldc, long long ldr, int M, int N) {
+  const int vec = N / 4;
+  const long long total = (long long)M * vec;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int row = (int)(i / vec), col = (int)(i - (long long)row * vec) * 4;
+    const float* src = ws + (long long)row * N + col;
+    float4 v[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (s < splits) v[s] = __ldcg(reinterpret_cast<const float4*>(src + s * split_stride));
+    float4 a = v[0];
+#pragma unroll
+    for (int s = 1; s < 8; ++s)
+      if (s < splits) { a.x += v[s].x; a.y += v[s].y; a.z += v[s].z; a.w += v[s].w; }
+    if constexpr (OUT_F32) {
+      float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(C) + row * ldc + col);
+      if constexpr (ACCUM) {
+        const float4 o = *dst;
+        a.x += o.x; a.y += o.y; a.z += o.z; a.w += o.w;
+      }
+      *dst = a;
+    } else {
+      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + row * ldc + col;
+      const __nv_bfloat16* add = ACCUM ? dst : R ? R + row * ldr + col : nullptr;
+      if (add) {
+        const uint2 o = *reinterpret_cast<const uint2*>(add);
+        a.x += __uint_as_float(o.x << 16);
+        a.y += __uint_as_float(o.x & 0xffff0000u);
+        a.z += __uint_as_float(o.y << 16);
+        a.w += __uint_as_float(o.y & 0xffff0000u);
+      }
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), h = __floats2bfloat162_rn(a.z, a.w);
+      *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo),
+                                                  *reinterpret_cast<const uint32_t*>(&h));
+    }
+  }
+}
+
+// One launch of the product kernel; `splits` > 1: `C` is the fp32 workspace.
+template <int BN>
+static int launch(const void* A, const void* B, void* C, const void* residual, int M, int N, int K,
+                  long long lda, long long ldb, long long ldc, long long ldr, bool a_mn, bool b_mn,
+                  bool out_fp32, bool accumulate, int splits, int max_ctas, cudaStream_t stream) {
+  CUtensorMap tmA, tmB, tmC;
+  // the tensor-map encoder is a driver call: make sure this thread (it may be an autograd
+  // worker) has the device's primary context bound
+  tc::bind_context_once();
+  Params p;
+  p.C = C;
+  p.R = residual;
+  p.ldc = ldc;
+  p.ldr = ldr;
+  p.M = M;
+  p.N = N;
+  p.K = K;
+  p.tiles_m = (M + BM - 1) / BM;
+  p.tiles_n = (N + BN - 1) / BN;
+  p.splits = splits;
+  p.split_rows = p.tiles_m * BM;
+  const long long items = (long long)p.tiles_m * p.tiles_n * splits;
+  int grid = sm_count();
+  if (grid > items) grid = (int)items;
+  if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
+  if (a_mn ? make_map(&tmA, A, K, M, lda, 64, BK) : make_map(&tmA, A, M, K, lda, BK, BM))
+    return 1003;
+  if (b_mn ? make_map(&tmB, B, K, N, ldb, 64, BK) : make_map(&tmB, B, N, K, ldb, BK, BN))
+    return 1004;
+  if (make_c_map(&tmC, C, splits > 1 ? splits * p.split_rows : M, N, ldc, out_fp32)) return 1008;
+  Kernel kernel = pick<BN>(a_mn, b_mn, out_fp32, accumulate);
+  if (!tc::ensure_dynamic_smem((const void*)kernel, Tile<BN>::SMEM_BYTES)) return 1005;
+  kernel<<<grid, kThreads, Tile<BN>::SMEM_BYTES, stream>>>(tmA, tmB, tmC, p);
+  return (int)cudaGetLastError();
+}
+
+static int check_args(const void* A, const void* B, const void* C, const void* residual, int N,
+                      long long lda, long long ldb, long long ldc, long long ldr, bool out_fp32,
+                      bool accumulate) {
+  // argument errors get codes of their own (1001..1008) so that they cannot be mistaken
+  // for a CUDA error
+  if ((lda % 8) || (ldb % 8) || (ldc % (out_fp32 ? 4 : 8)) || (N % 8)) return 1001;
+  if (((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15)) return 1002;
+  if (residual && (out_fp32 || accumulate || (ldr % 8) || ((uintptr_t)residual & 15))) return 1001;
+  return 0;
 }
 
 }  // namespace gemm
@@ -281,42 +404,60 @@ int bcom_gemm_bf16_ex(const void* A, const void* B, void* C, const void* residua
                       void* stream) {
   using namespace gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  // argument errors get codes of their own (1001..1005) so that they cannot be mistaken
-  // for a CUDA error
-  if ((lda % 8) || (ldb % 8) || (ldc % (out_fp32 ? 4 : 8)) || (N % 8)) return 1001;
-  if (((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15)) return 1002;
-  if (residual && (out_fp32 || accumulate || (ldr % 8) || ((uintptr_t)residual & 15))) return 1001;
+  if (const int rc = check_args(A, B, C, residual, N, lda, ldb, ldc, ldr, out_fp32 != 0,
+                                accumulate != 0))
+    return rc;
   (void)cudaGetLastError();  // do not inherit an error left behind by an earlier call
-  CUtensorMap tmA, tmB, tmC;
-  // the tensor-map encoder is a driver call: make sure this thread (it may be an autograd
-  // worker) has the device's primary context bound
-  tc::bind_context_once();
-  Params p;
-  p.C = C;
-  p.R = residual;
-  p.ldc = ldc;
-  p.ldr = ldr;
-  p.M = M;
-  p.N = N;
-  p.K = K;
-  p.tiles_m = (M + BM - 1) / BM;
-  p.tiles_n = (N + BN - 1) / BN;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int tiles = p.tiles_m * p.tiles_n;
-  int grid = tiles;
-  if (grid > sms) grid = sms;
-  if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  if (a_mn_major ? make_map(&tmA, A, K, M, lda, 64, BK) : make_map(&tmA, A, M, K, lda, BK, BM))
-    return 1003;
-  if (b_mn_major ? make_map(&tmB, B, K, N, ldb, 64, BK)
-                 : make_map(&tmB, B, N, K, ldb, BK, BN))
-    return 1004;
-  if (make_c_map(&tmC, C, M, N, ldc, out_fp32 != 0)) return 1008;
-  Kernel kernel = pick(a_mn_major != 0, b_mn_major != 0, out_fp32 != 0, accumulate != 0);
-  if (!tc::ensure_dynamic_smem((const void*)kernel, SMEM_BYTES)) return 1005;
-  kernel<<<grid, kThreads, SMEM_BYTES, (cudaStream_t)stream>>>(tmA, tmB, tmC, p);
+  return launch<256>(A, B, C, residual, M, N, K, lda, ldb, ldc, ldr, a_mn_major != 0,
+                     b_mn_major != 0, out_fp32 != 0, accumulate != 0, 1, max_ctas,
+                     (cudaStream_t)stream);
+}
+
+// fp32 elements of workspace that bcom_gemm_bf16_split needs (0 for splits <= 1)
+long long bcom_gemm_split_workspace(int M, int N, int splits) {
+  return splits <= 1 ? 0 : (long long)splits * ((M + 127) / 128 * 128) * N;
+}
+
+// The same product on 128x128 tiles with K shared out among `splits` (1..8) work items per tile,
+// for shapes with few tiles: 128 tokens through a 4096 x 4096 projection are 16 tiles of 128x256,
+// i.e. 16 of 148 SMs fetching the weights in 64 serial k-blocks each.  splits > 1: the partial
+// tiles go to `workspace` (private to the call until it has run, 16-byte aligned) and a second
+// kernel adds them up in ascending order.  `splits` must not exceed the 64-wide k-blocks.
+int bcom_gemm_bf16_split(const void* A, const void* B, void* C, const void* residual, int M, int N,
+                         int K, long long lda, long long ldb, long long ldc, long long ldr,
+                         int a_mn_major, int b_mn_major, int out_fp32, int accumulate, int splits,
+                         void* workspace, void* stream) {
+  using namespace gemm;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (const int rc = check_args(A, B, C, residual, N, lda, ldb, ldc, ldr, out_fp32 != 0,
+                                accumulate != 0))
+    return rc;
+  if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) return (int)cudaErrorInvalidValue;
+  (void)cudaGetLastError();
+  cudaStream_t st = (cudaStream_t)stream;
+  if (splits == 1)
+    return launch<128>(A, B, C, residual, M, N, K, lda, ldb, ldc, ldr, a_mn_major != 0,
+                       b_mn_major != 0, out_fp32 != 0, accumulate != 0, 1, 0, st);
+  if (!workspace || ((uintptr_t)workspace & 15)) return 1002;
+  const int rc = launch<128>(A, B, workspace, nullptr, M, N, K, lda, ldb, N, 0, a_mn_major != 0,
+                             b_mn_major != 0, true, false, splits, 0, st);
+  if (rc) return rc;
+  const long long stride = (long long)((M + BM - 1) / BM * BM) * N;
+  const long long work = ((long long)M * (N / 4) + 255) / 256;
+  const int grid = (int)(work < 4LL * sm_count() ? work : 4LL * sm_count());
+  const float* ws = (const float*)workspace;
+  const __nv_bfloat16* R = (const __nv_bfloat16*)residual;
+  if (out_fp32) {
+    if (accumulate)
+      split_sum_kernel<true, true><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, ldc, ldr, M, N);
+    else
+      split_sum_kernel<true, false><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, ldc, ldr, M, N);
+  } else {
+    if (accumulate)
+      split_sum_kernel<false, true><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, ldc, ldr, M, N);
+    else
+      split_sum_kernel<false, false><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, ldc, ldr, M, N);
+  }
   return (int)cudaGetLastError();
 }
 

@@ -6,6 +6,7 @@ reference trainer's model is plain ``nn.Linear``
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -31,6 +32,10 @@ def _get():
                                            ci, vp]
             lib.bcom_gemm_bf16_ex.argtypes = [vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci, ci,
                                               ci, ci, ci, vp]
+            lib.bcom_gemm_bf16_split.argtypes = [vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci,
+                                                 ci, ci, ci, ci, vp, vp]
+            lib.bcom_gemm_split_workspace.argtypes = [ci, ci, ci]
+            lib.bcom_gemm_split_workspace.restype = ll
             lib.bcom_gemm_status.argtypes = [ctypes.POINTER(ctypes.c_uint * 4), ci]
         _lib = lib if lib is not None else False
     return _lib or None
@@ -69,7 +74,7 @@ def available() -> bool:
 
 def variant() -> str:
     """The kernel that ``gemm`` launches: "1cta", "2cta" (CTA pairs, 256x256 tiles,
-    ``tcgen05.mma.cta_group::2``) or "auto" (default: by shape, see ``_use_pair``).  Initialised
+    ``tcgen05.mma.cta_group::2``) or "auto" (default: by shape, see ``_plan``).  Initialised
     from ``BITSCOM_GEMM``."""
     global _variant
     if _variant is None:
@@ -82,12 +87,41 @@ def variant() -> str:
     return _variant
 
 
-def _use_pair(M: int, N: int) -> bool:
-    """More than one wave of 128x256 tiles: CTA pairs, which read half as much of B per SM and
-    keep the tensor pipe busier (4096 x 22016 x 4096: 548 -> 508 us, its weight gradient 661 ->
-    601 us).  Up to one wave the pairs' 256-row tiles leave more of the chip idle than they
-    save (1024 x 4096 x 4096: 26.7 -> 28.7 us)."""
-    return -(-M // 128) * -(-N // 256) > 148 and _get2() is not None
+_SMS = 148
+
+
+@functools.lru_cache(maxsize=4096)
+def _plan(M: int, N: int, K: int, a_mn_major: bool = False, max_ctas: int = 0) -> int:
+    """Which kernel "auto" runs: -1 CTA pairs, 0 the one-CTA kernel on 128x256 tiles, S >= 1 its
+    128x128 form with K shared out among S work items per tile.
+
+    * More than one wave of 128x256 tiles: pairs, which read half as much of B per SM and keep the
+      tensor pipe busier (4096 x 22016 x 4096: 548 -> 508 us, its weight gradient 661 -> 601 us).
+      With fewer than 8 k-blocks C's traffic is all there is and the pairs' hand-offs show
+      (12288 x 4096 from 128 tokens: 89.6 -> 92.7 us).  Weight gradients take pairs from half a
+      wave on (3072 x 1024 x 4096: 29.3 -> 26.5 us); other products do not (4096 x 1024 x 4096:
+      25.3 -> 26.1 us).
+    * Fewer tiles: the 128x128 form where its tiles fit one wave (512 x 4096 x 4096: 23.9 -> 21.7
+      us), with the S that is cheapest by this model, in units of one 128x128 k-block (0.27 us):
+      waves x k-blocks per item, plus 16 for the second launch and the workspace's bytes at 6 TB/s
+      (128 x 4096 x 4096: 23.1 us as 16 tiles, 11.5 us with S = 4; 128 x 4096 x 22016: 121 ->
+      36 us).  A 128x256 k-block costs 1.33 units."""
+    kb = -(-K // 64)
+    rows = -(-M // 128)
+    tiles = rows * -(-N // 256)
+    if max_ctas != 1 and kb >= 8 and (tiles > _SMS or (a_mn_major and 2 * tiles > _SMS)) \
+            and _get2() is not None:
+        return -1
+    if tiles > _SMS or max_ctas > 0:
+        return 0
+    small = rows * -(-N // 128)
+
+    def cost(splits: int) -> float:
+        c = -(-small * splits // _SMS) * -(-kb // splits)
+        return c + (16 + 4.9e-6 * splits * rows * 128 * N if splits > 1 else 0)
+
+    best = min(range(1, min(8, kb) + 1), key=cost)
+    return best if cost(best) < 1.33 * kb else 0
 
 
 def set_variant(name: str) -> str:
@@ -207,9 +241,20 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False,
                                  or residual.dtype != torch.bfloat16):
         raise ValueError("bad residual tensor")
     kind = variant()
-    pair = max_ctas != 1 and _use_pair(M, N) if kind == "auto" else kind == "2cta"
-    launch = _get2().bcom_gemm2_bf16_ex if pair else lib.bcom_gemm_bf16_ex
+    plan = _plan(M, N, K, a_mn_major, max_ctas) if kind == "auto" else 0 if kind == "1cta" else -1
     with _native.on_device(a.device):
+        if plan > 0:
+            ws = None
+            if plan > 1:
+                ws = torch.empty(lib.bcom_gemm_split_workspace(M, N, plan), dtype=torch.float32,
+                                 device=a.device)
+            check(lib.bcom_gemm_bf16_split(
+                ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K, a.stride(0), b.stride(0),
+                out.stride(0), 0 if residual is None else residual.stride(0), int(a_mn_major),
+                int(b_mn_major), int(out.dtype == torch.float32), int(accumulate), plan, ptr(ws),
+                stream_ptr(a.device)), "bcom_gemm_bf16_split", launches=1 + (plan > 1))
+            return out
+        launch = lib.bcom_gemm_bf16_ex if plan == 0 else _get2().bcom_gemm2_bf16_ex
         check(launch(
             ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K, a.stride(0), b.stride(0),
             out.stride(0), 0 if residual is None else residual.stride(0),

@@ -42,6 +42,14 @@ int main() {
     }
     checked += 2;
   }
+  // shares of K: in order, without gaps, none empty
+  for (int kb = 1; kb <= 200; ++kb)
+    for (int splits = 1; splits <= 8 && splits <= kb; ++splits)
+      for (int i = 0; i < splits; ++i) {
+        const int from = gemm_sched::split_begin(kb, splits, i);
+        const int to = gemm_sched::split_begin(kb, splits, i + 1);
+        if (from >= to || (i == 0 && from != 0) || (i + 1 == splits && to != kb)) return 8;
+      }
   std::printf("ok: %d schedules cover their outputs exactly once\n", checked);
   return 0;
 }

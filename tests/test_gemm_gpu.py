@@ -147,6 +147,37 @@ def test_cta_pair_gemm(a_mn, b_mn, M, N, K):
     assert torch.equal(exact, _ref(ai, bi, a_mn, b_mn))
 
 
+@pytest.mark.parametrize("a_mn", [False, True])
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("splits,M,N,K", [(1, 128, 128, 64), (1, 136, 264, 328), (2, 200, 264, 2056),
+                                          (3, 8, 8, 520), (5, 264, 136, 4104), (8, 128, 128, 512),
+                                          (8, 77, 200, 1000)])
+def test_gemm_split_k(monkeypatch, splits, a_mn, b_mn, M, N, K):
+    """The 128x128 form, K shared out among 1..8 items per tile, with ragged edges and uneven
+    shares, strided output and every output form; exact on small integers (all sums below 2^24)."""
+    if (a_mn and M % 8):
+        pytest.skip("row stride must stay 16-byte aligned")
+    monkeypatch.setattr(G, "_plan", lambda *a: splits)
+    ai = torch.randint(-3, 4, (K, M) if a_mn else (M, K), device="cuda").to(torch.bfloat16)
+    bi = torch.randint(-3, 4, (K, N) if b_mn else (N, K), device="cuda").to(torch.bfloat16)
+    ref = _ref(ai, bi, a_mn, b_mn)
+    kw = dict(a_mn_major=a_mn, b_mn_major=b_mn)
+    wide = torch.full((M, N + 16), 7.0, device="cuda")
+    acc = G.gemm(ai, bi, out=wide[:, 8:8 + N], **kw)
+    assert torch.equal(acc, ref)
+    G.gemm(ai, bi, out=acc, accumulate=True, **kw)
+    assert torch.equal(acc, 2 * ref)
+    assert (wide[:, :8] == 7).all() and (wide[:, 8 + N:] == 7).all()
+    res = torch.randint(-3, 4, (M, N), device="cuda").to(torch.bfloat16)
+    assert torch.equal(G.gemm(ai, bi, residual=res, **kw), (ref + res.float()).to(torch.bfloat16))
+    out = G.gemm(ai, bi, **kw)
+    assert torch.equal(out, ref.to(torch.bfloat16))
+    old = out.float()
+    G.gemm(ai, bi, out=out, accumulate=True, **kw)
+    assert torch.equal(out, (old + ref).to(torch.bfloat16))
+    G.check_status()
+
+
 def test_gemm_throughput_report():
     M = N = K = 8192
     a, b = _mk(M, K, 1), _mk(N, K, 2)
