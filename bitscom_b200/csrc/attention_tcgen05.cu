@@ -380,101 +380,110 @@ attention_fwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_q,    // b
 
   if (warp == 4) {
     // ------------------------------- issuer -------------------------------------------
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = tc::make_idesc_bf16(BQ, BKF, false, false);
-      constexpr uint32_t idesc_o = tc::make_idesc_bf16(BQ, HD, false, true);
-      const uint32_t aQ = tc::smem_u32(sQ), aK0 = tc::smem_u32(sK0), aV0 = tc::smem_u32(sV0),
-                     aP = tc::smem_u32(sP);
-      bool ok = true;
-      auto wait = [&](uint64_t* bar, uint32_t parity, unsigned code) {
-        if (ok && !tc::mbar_wait(bar, parity, kBudgetNs)) {
-          ok = false;
+    // The whole warp walks the loop, one elected lane issues copies and MMAs: descriptors and
+    // addresses stay in uniform registers and cost one add each.
+    constexpr uint32_t idesc_s = tc::make_idesc_bf16(BQ, BKF, false, false);
+    constexpr uint32_t idesc_o = tc::make_idesc_bf16(BQ, HD, false, true);
+    constexpr uint32_t hi = tc::desc_hi(1024);
+    const uint32_t q_lo = tc::desc_lo(tc::smem_u32(sQ), 16), k_lo = tc::desc_lo(tc::smem_u32(sK0), 16),
+                   v_lo = tc::desc_lo(tc::smem_u32(sV0), BKF * 128),
+                   p_lo = tc::desc_lo(tc::smem_u32(sP), 16);
+    bool ok = true;
+    auto wait = [&](uint64_t* bar, uint32_t parity, unsigned code) {
+      if (ok && !tc::mbar_wait_warp(bar, parity, kBudgetNs)) {
+        ok = false;
+        if (lane == 0) {
           sh->abort = 1;
           record_fail(code);
         }
-      };
-      auto load_k = [&](int j) {
-        uint64_t* bar = &sh->bar_k[j & 1];
+      }
+    };
+    auto load_kv = [&](uint8_t* base, uint64_t* bars, int col, int j) {
+      if (tc::elect_one()) {
+        uint64_t* bar = &bars[j & 1];
         tc::mbar_expect_tx(bar, K_BYTES);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c)
-          tc::tma_load_2d(sK0 + (j & 1) * K_BYTES + c * BKF * 128, &tm_kv, bar, k_col + 64 * c,
+          tc::tma_load_2d(base + (j & 1) * K_BYTES + c * BKF * 128, &tm_kv, bar, col + 64 * c,
                           b * p.seq + j * BKF);
-      };
-      auto load_v = [&](int j) {
-        uint64_t* bar = &sh->bar_v[j & 1];
-        tc::mbar_expect_tx(bar, K_BYTES);
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c)
-          tc::tma_load_2d(sV0 + (j & 1) * K_BYTES + c * BKF * 128, &tm_kv, bar, v_col + 64 * c,
-                          b * p.seq + j * BKF);
-      };
-      auto issue_qk = [&](int j) {
-        const uint32_t aK = aK0 + (j & 1) * K_BYTES;
+      }
+      __syncwarp();
+    };
+    auto issue_qk = [&](int j) {
+      const uint32_t k = k_lo + (j & 1) * (K_BYTES >> 4);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks)
-          tc::umma_bf16(tmem + (j & 1) * 64, desc_kmajor(aQ, BQ, ks), desc_kmajor(aK, BKF, ks),
-                        idesc_s, ks != 0);
+          tc::umma_bf16_lo<1>(tmem + (j & 1) * 64,
+                              q_lo + (ks >> 2) * (BQ * 128 >> 4) + (ks & 3) * 2, hi,
+                              k + (ks >> 2) * (BKF * 128 >> 4) + (ks & 3) * 2, hi, idesc_s,
+                              ks != 0);
         tc::umma_commit(&sh->bar_s[j & 1]);
-      };
-      auto issue_pv = [&](int j) {
-        const uint32_t aV = aV0 + (j & 1) * K_BYTES;
+      }
+      __syncwarp();
+    };
+    auto issue_pv = [&](int j) {
+      const uint32_t v = v_lo + (j & 1) * (K_BYTES >> 4);
+      if (tc::elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < BKF / 16; ++ks)
-          tc::umma_bf16(tO, desc_kmajor(aP, BQ, ks), desc_mnmajor(aV, BKF, ks), idesc_o,
-                        (j != 0) || (ks != 0));
+          tc::umma_bf16_lo<1>(tO, p_lo + ks * 2, hi, v + ks * (16 * 128 >> 4), hi, idesc_o,
+                              (j != 0) || (ks != 0));
         tc::umma_commit(&sh->bar_o);
-      };
+      }
+      __syncwarp();
+    };
 
+    if (tc::elect_one()) {
       tc::mbar_expect_tx(&sh->bar_q, Q_BYTES);
 #pragma unroll
       for (int c = 0; c < HD / 64; ++c)
         tc::tma_load_2d(sQ + c * BQ * 128, &tm_q, &sh->bar_q, q_col + 64 * c, row0);
-      load_k(0);
-      load_v(0);
-      if (n > 1) {
-        load_k(1);
-        load_v(1);
-      }
-      wait(&sh->bar_q, 0, 21);
-      wait(&sh->bar_k[0], 0, 22);
-      if (ok) {
-        tc::tc_fence_after_sync();
-        issue_qk(0);
-      }
-      if (n > 1) {
-        wait(&sh->bar_k[1], 0, 22);
-        if (ok) {
-          tc::tc_fence_after_sync();
-          issue_qk(1);
-        }
-      }
-      for (int j = 0; j < n && ok; ++j) {
-        const uint32_t par2 = (uint32_t)(j >> 1) & 1u;
-        if (j + 2 < n) {  // K buffer j & 1 is free once QK_j has completed
-          wait(&sh->bar_s[j & 1], par2, 23);
-          if (ok) load_k(j + 2);
-        }
-        if (j >= 1 && j + 1 < n) {  // V buffer (j + 1) & 1 is free once PV_{j-1} has completed
-          wait(&sh->bar_o, (uint32_t)(j - 1) & 1u, 24);
-          if (ok) load_v(j + 1);
-        }
-        wait(&sh->bar_p, (uint32_t)j & 1u, 25);  // P_j written, S_j consumed, O rescaled
-        wait(&sh->bar_v[j & 1], par2, 26);
-        if (!ok) break;
-        tc::tc_fence_after_sync();
-        issue_pv(j);
-        if (j + 2 < n) {
-          wait(&sh->bar_k[j & 1], (uint32_t)((j + 2) >> 1) & 1u, 22);
-          if (!ok) break;
-          tc::tc_fence_after_sync();
-          issue_qk(j + 2);
-        }
-      }
-      // every MMA issued must have finished before TMEM is handed back
-      if (ok && n > 0) wait(&sh->bar_o, (uint32_t)(n - 1) & 1u, 27);
     }
     __syncwarp();
+    load_kv(sK0, sh->bar_k, k_col, 0);
+    load_kv(sV0, sh->bar_v, v_col, 0);
+    if (n > 1) {
+      load_kv(sK0, sh->bar_k, k_col, 1);
+      load_kv(sV0, sh->bar_v, v_col, 1);
+    }
+    wait(&sh->bar_q, 0, 21);
+    wait(&sh->bar_k[0], 0, 22);
+    if (ok) {
+      tc::tc_fence_after_sync();
+      issue_qk(0);
+    }
+    if (n > 1) {
+      wait(&sh->bar_k[1], 0, 22);
+      if (ok) {
+        tc::tc_fence_after_sync();
+        issue_qk(1);
+      }
+    }
+    for (int j = 0; j < n && ok; ++j) {
+      const uint32_t par2 = (uint32_t)(j >> 1) & 1u;
+      if (j + 2 < n) {  // K buffer j & 1 is free once QK_j has completed
+        wait(&sh->bar_s[j & 1], par2, 23);
+        if (ok) load_kv(sK0, sh->bar_k, k_col, j + 2);
+      }
+      if (j >= 1 && j + 1 < n) {  // V buffer (j + 1) & 1 is free once PV_{j-1} has completed
+        wait(&sh->bar_o, (uint32_t)(j - 1) & 1u, 24);
+        if (ok) load_kv(sV0, sh->bar_v, v_col, j + 1);
+      }
+      wait(&sh->bar_p, (uint32_t)j & 1u, 25);  // P_j written, S_j consumed, O rescaled
+      wait(&sh->bar_v[j & 1], par2, 26);
+      if (!ok) break;
+      tc::tc_fence_after_sync();
+      issue_pv(j);
+      if (j + 2 < n) {
+        wait(&sh->bar_k[j & 1], (uint32_t)((j + 2) >> 1) & 1u, 22);
+        if (!ok) break;
+        tc::tc_fence_after_sync();
+        issue_qk(j + 2);
+      }
+    }
+    // every MMA issued must have finished before TMEM is handed back
+    if (ok && n > 0) wait(&sh->bar_o, (uint32_t)(n - 1) & 1u, 27);
   } else {
     // ------------------------------- softmax warps ------------------------------------
     const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
@@ -887,6 +896,386 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box {64, 1
   }
 }
 
+// ---------------------------------------------------------------------------
+// backward, software-pipelined
+// ---------------------------------------------------------------------------
+// Same products as attention_bwd_kernel (everything transposed, rows = keys), but no role waits
+// for another one's whole step.  In the kernel above one thread issues the MMAs, everybody
+// waits for them, everybody does the element-wise part, and the next Q / dO tiles are requested
+// only after the last MMA: 13 k cycles per 128 x 128 block where the five products take 2.6 k.
+//   warps 0-7   softmax: P^T (bf16) goes back into tensor memory, over the S^T columns the warp
+//               has just read, and is the A operand of dV from there; dS^T goes to shared memory
+//   warps 8-11  dQ: tensor memory -> staging -> bulk reductions into the fp32 accumulator, each
+//               warp its own 32 rows, in two halves of HD / 2 columns
+//   warp 12     issuer, warp 13 loader
+// Order on the tensor pipe: S_0 dP_0 | dV_0 S_1 dQ_0 dK_0 dP_1 | dV_1 S_2 dQ_1 dK_1 dP_2 | ...
+// so the exponentials of block i + 1 run under dQ_i dK_i dP_{i+1}, and dS_{i+1} under dV_{i+1}
+// S_{i+2}.  P^T in tensor memory leaves the shared memory for two Q and two dO tiles; dQ is
+// staged in the dO tile of its own block, which nobody needs after dV_i.
+// Why each buffer may be written when it is:
+//   S (and P over it)   S_{i+1} is issued after dV_i has completed (dv_done)
+//   dP (and dQ over it) dQ_i after ds_full(i) (dP_i read), dP_{i+1} after dq_drained(i)
+//   dS                  written after dp_full(i+1), whose commit follows dQ_i and dK_i
+//   Q, lse, delta [s]   loaded after q_empty (dK_i complete, hence ds_full(i))
+//   dO [s]              staging after dq_full(i), whose commit follows dV_i; loaded after do_empty
+//                       (the reductions have read the staging tile)
+// Measured (B2 S2048 H32 D128): 391 -> BWD_US us; (B8 S1024 H16 D64): 189 -> BWD64_US us.
+constexpr int kBwdPipeThreads = 14 * 32;
+
+struct BwdPipeShared {
+  float lse[2][BQ], delta[2][BQ];
+  uint64_t kv_full, q_full[2], do_full[2], q_empty[2], do_empty[2];
+  uint64_t s_full, dp_full, p_full, ds_full, dv_done, dq_full, dq_drained, fin;
+  uint32_t tmem_base;
+  volatile int abort;
+};
+
+template <int HD> struct BwdPipe {
+  static constexpr int TILE = 128 * HD * 2;
+  // no slack for manual alignment: the kernel checks the dynamic window (see FwdPipe)
+  static constexpr int SMEM = 6 * TILE + TILE_SQ + sizeof(BwdPipeShared);
+};
+
+template <int HD>
+__global__ void __launch_bounds__(kBwdPipeThreads, 1)
+attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {64, 128}
+                               const __grid_constant__ CUtensorMap tm_do,   // box {64, 128}
+                               const __grid_constant__ CUtensorMap tm_dq,   // fp32, box {32, 32}
+                               const BwdParams p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  constexpr int TILE = BwdPipe<HD>::TILE;
+  uint8_t* sK = smem;
+  uint8_t* sV = sK + TILE;
+  uint8_t* sQ = sV + TILE;        // two stages
+  uint8_t* sDO = sQ + 2 * TILE;   // two stages
+  uint8_t* sDS = sDO + 2 * TILE;
+  BwdPipeShared* sh = reinterpret_cast<BwdPipeShared*>(sDS + TILE_SQ);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if ((tc::smem_u32(smem) & 1023u) != 0u) {  // same answer in every thread of the CTA
+    if (tid == 0) record_fail(40);
+    return;
+  }
+  const int kblocks = p.seq / BKB;
+  // key blocks with the most query blocks first, over all heads: the last ones to start are short
+  const int heads = p.batch * p.heads;
+  const int kb = (int)blockIdx.x / heads;
+  const int bh = (int)blockIdx.x - kb * heads;
+  const int h = bh % p.heads, b = bh / p.heads;
+  const int H = p.heads * HD;
+  const int key0 = b * p.seq + kb * BKB;
+  const int q_col = h * HD, k_col = H + h * HD, v_col = 2 * H + h * HD;
+  const int n = kblocks - kb;  // query blocks kb .. kblocks-1 (BQ == BKB)
+
+  if (tid == 0) {
+    tc::mbar_init(&sh->kv_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&sh->q_full[i], 1);
+      tc::mbar_init(&sh->do_full[i], 1);
+      tc::mbar_init(&sh->q_empty[i], 1);
+      tc::mbar_init(&sh->do_empty[i], 4);
+    }
+    tc::mbar_init(&sh->s_full, 1);
+    tc::mbar_init(&sh->dp_full, 1);
+    tc::mbar_init(&sh->p_full, 8);
+    tc::mbar_init(&sh->ds_full, 8);
+    tc::mbar_init(&sh->dv_done, 1);
+    tc::mbar_init(&sh->dq_full, 1);
+    tc::mbar_init(&sh->dq_drained, 4);
+    tc::mbar_init(&sh->fin, 1);
+    sh->abort = 0;
+    tc::fence_mbar_init();
+  }
+  if (warp == 12) tc::tmem_alloc(&sh->tmem_base, 512);
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  tc::tc_fence_after_sync();
+  const uint32_t tmem = sh->tmem_base;
+  const uint32_t tS = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 256 + HD;
+  const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+
+  bool ok = true;
+  // every lane of a warp waits; the verdict is uniform
+  auto wait = [&](uint64_t* bar, uint32_t parity, unsigned code) {
+    if (ok && !tc::mbar_wait_warp(bar, parity, kBudgetNs)) {
+      ok = false;
+      if (lane == 0) {
+        sh->abort = 1;
+        record_fail(code);
+      }
+    }
+    return ok;
+  };
+  auto arrive = [&](uint64_t* bar) {  // once per warp, after every lane's accesses
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(bar);
+  };
+
+  if (warp < 8) {
+    // ------------------------------- softmax ------------------------------------------
+    const int row = ((warp & 3) << 5) | lane;  // key row
+    const int half = warp >> 2;                // query columns [64 half, 64 half + 64)
+    for (int i = 0; i < n; ++i) {
+      const uint32_t par = (uint32_t)i & 1u, par2 = (uint32_t)(i >> 1) & 1u;
+      const float* lse = sh->lse[i & 1] + half * 64;
+      const float* delta = sh->delta[i & 1] + half * 64;
+      if (!wait(&sh->q_full[i & 1], par2, 41) || !wait(&sh->s_full, par, 42)) break;
+      tc::tc_fence_after_sync();
+      float pt[64];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r[32];
+        tc::tmem_ld_32x32(tS + lane_addr + half * 64 + c * 32, r);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          const float4 l = *reinterpret_cast<const float4*>(lse + c * 32 + v * 4);
+          const float ls[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            pt[c * 32 + v * 4 + u] =
+                ex2_fast(__uint_as_float(r[v * 4 + u]) * p.scale_log2 - ls[u]);
+        }
+      }
+      if (i == 0) {  // the block on the diagonal: query >= key
+        const int first = row - half * 64;  // columns before it are masked
+#pragma unroll
+        for (int c = 0; c < 64; ++c)
+          if (c < first) pt[c] = 0.0f;
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t w[16];
+#pragma unroll
+        for (int v = 0; v < 16; ++v) w[v] = pack_bf16(pt[c * 32 + 2 * v], pt[c * 32 + 2 * v + 1]);
+        tc::tmem_st_32x16(tS + lane_addr + half * 64 + c * 16, w);
+      }
+      tc::tmem_wait_st();
+      tc::tc_fence_before_sync();
+      arrive(&sh->p_full);
+
+      if (!wait(&sh->dp_full, par, 43)) break;
+      tc::tc_fence_after_sync();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r[32];
+        tc::tmem_ld_32x32(tDP + lane_addr + half * 64 + c * 32, r);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const float4 d0 = *reinterpret_cast<const float4*>(delta + c * 32 + v * 8);
+          const float4 d1 = *reinterpret_cast<const float4*>(delta + c * 32 + v * 8 + 4);
+          const float dl[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+          float ds[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            ds[u] = pt[c * 32 + v * 8 + u] * (__uint_as_float(r[v * 8 + u]) - dl[u]) * p.scale;
+          *reinterpret_cast<uint4*>(sDS + half * 128 * 128 + swz(row, c * 4 + v)) =
+              make_uint4(pack_bf16(ds[0], ds[1]), pack_bf16(ds[2], ds[3]),
+                         pack_bf16(ds[4], ds[5]), pack_bf16(ds[6], ds[7]));
+        }
+      }
+      tc::fence_proxy_async();       // dS^T is visible to the MMA
+      tc::tc_fence_before_sync();    // dP^T has been read
+      arrive(&sh->ds_full);
+    }
+    // ---- dK, dV rows (thread t <-> key row t; the two halves split the columns) ----
+    if (wait(&sh->fin, 0, 44)) {
+      tc::tc_fence_after_sync();
+      __nv_bfloat16* dk = p.dqkv + (size_t)(key0 + row) * 3 * H + k_col;
+      __nv_bfloat16* dv = p.dqkv + (size_t)(key0 + row) * 3 * H + v_col;
+#pragma unroll 1
+      for (int c = half * (HD / 64); c < (half + 1) * (HD / 64); ++c) {
+#pragma unroll 1
+        for (int t = 0; t < 2; ++t) {
+          uint32_t r[32];
+          tc::tmem_ld_32x32((t ? tDV : tDK) + lane_addr + c * 32, r);
+          tc::tmem_wait_ld();
+          uint4* dst = reinterpret_cast<uint4*>((t ? dv : dk) + c * 32);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            dst[u] = make_uint4(
+                pack_bf16(__uint_as_float(r[u * 8 + 0]), __uint_as_float(r[u * 8 + 1])),
+                pack_bf16(__uint_as_float(r[u * 8 + 2]), __uint_as_float(r[u * 8 + 3])),
+                pack_bf16(__uint_as_float(r[u * 8 + 4]), __uint_as_float(r[u * 8 + 5])),
+                pack_bf16(__uint_as_float(r[u * 8 + 6]), __uint_as_float(r[u * 8 + 7])));
+        }
+      }
+    }
+  } else if (warp < 12) {
+    // ------------------------------- dQ ------------------------------------------------
+    const int w = warp - 8;
+    constexpr int SUB = HD / 64;  // 32-column sub-tiles per half
+    for (int i = 0; i < n; ++i) {
+      uint8_t* stage = sDO + (i & 1) * TILE + w * (SUB * 4096);
+      const int qrow = b * p.seq + (kb + i) * BQ + w * 32;
+      if (!wait(&sh->dq_full, (uint32_t)i & 1u, 45)) break;
+      tc::tc_fence_after_sync();
+#pragma unroll 1
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t r[SUB][32];
+#pragma unroll
+        for (int c = 0; c < SUB; ++c)
+          tc::tmem_ld_32x32(tDP + lane_addr + hf * (HD / 2) + c * 32, r[c]);
+        tc::tmem_wait_ld();
+        if (hf == 1) {
+          tc::tc_fence_before_sync();
+          arrive(&sh->dq_drained);
+          if (lane == 0) tc::bulk_wait_group_read0();  // the first half has left the staging tile
+          __syncwarp();
+        }
+#pragma unroll
+        for (int c = 0; c < SUB; ++c)
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            *reinterpret_cast<uint4*>(stage + c * 4096 + swz(lane, u)) =
+                make_uint4(r[c][u * 4], r[c][u * 4 + 1], r[c][u * 4 + 2], r[c][u * 4 + 3]);
+        tc::fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+#pragma unroll
+          for (int c = 0; c < SUB; ++c)
+            tc::tma_reduce_add_2d(&tm_dq, stage + c * 4096, q_col + hf * (HD / 2) + c * 32, qrow);
+          tc::bulk_commit_group();
+        }
+      }
+      if (lane == 0) tc::bulk_wait_group_read0();
+      arrive(&sh->do_empty[i & 1]);
+    }
+    if (lane == 0) tc::bulk_wait_group0();  // the reductions are performed before the CTA exits
+    __syncwarp();
+  } else if (warp == 12) {
+    // ------------------------------- issuer ---------------------------------------------
+    constexpr uint32_t idesc_kk = tc::make_idesc_bf16(128, 128, false, false);  // both K-major
+    constexpr uint32_t idesc_kn = tc::make_idesc_bf16(128, HD, false, true);    // B MN-major
+    constexpr uint32_t idesc_nn = tc::make_idesc_bf16(128, HD, true, true);     // both MN-major
+    constexpr uint32_t hi = tc::desc_hi(1024);
+    constexpr uint32_t MN = 128 * 128;  // bytes between 64-column chunks of an MN-major operand
+    const uint32_t aK = tc::smem_u32(sK), aV = tc::smem_u32(sV), aQ = tc::smem_u32(sQ),
+                   aDO = tc::smem_u32(sDO), aDS = tc::smem_u32(sDS);
+    const uint32_t k_k = tc::desc_lo(aK, 16), v_k = tc::desc_lo(aV, 16), k_n = tc::desc_lo(aK, MN),
+                   ds_k = tc::desc_lo(aDS, 16), ds_n = tc::desc_lo(aDS, MN);
+    // k-step ks of a K-major operand (64-column chunks 16 KiB apart) and of an MN-major one
+    auto kstep = [](int ks) { return (uint32_t)((ks >> 2) * (MN >> 4) + (ks & 3) * 2); };
+    auto nstep = [](int ks) { return (uint32_t)(ks * (16 * 128 >> 4)); };
+    auto issue_s = [&](int i) {
+      const uint32_t q = tc::desc_lo(aQ + (i & 1) * TILE, 16);
+      if (tc::elect_one()) {
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks)
+          tc::umma_bf16_lo<1>(tS, k_k + kstep(ks), hi, q + kstep(ks), hi, idesc_kk, ks != 0);
+        tc::umma_commit(&sh->s_full);
+      }
+      __syncwarp();
+    };
+    auto issue_dp = [&](int i) {
+      const uint32_t g = tc::desc_lo(aDO + (i & 1) * TILE, 16);
+      if (tc::elect_one()) {
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks)
+          tc::umma_bf16_lo<1>(tDP, v_k + kstep(ks), hi, g + kstep(ks), hi, idesc_kk, ks != 0);
+        tc::umma_commit(&sh->dp_full);
+      }
+      __syncwarp();
+    };
+    if (wait(&sh->kv_full, 0, 46) && wait(&sh->q_full[0], 0, 47)) {
+      tc::tc_fence_after_sync();
+      issue_s(0);
+      if (wait(&sh->do_full[0], 0, 48)) {
+        tc::tc_fence_after_sync();
+        issue_dp(0);
+      }
+    }
+    for (int i = 0; i < n && ok; ++i) {
+      const uint32_t par = (uint32_t)i & 1u;
+      const int s = i & 1, sn = (i + 1) & 1;
+      const uint32_t parn = (uint32_t)((i + 1) >> 1) & 1u;
+      if (!wait(&sh->p_full, par, 49)) break;
+      tc::tc_fence_after_sync();
+      {
+        const uint32_t g = tc::desc_lo(aDO + s * TILE, MN);
+        if (tc::elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < BQ / 16; ++ks)
+            tc::umma_bf16_ta(tDV, tS + (ks >> 2) * 64 + (ks & 3) * 8, g + nstep(ks), hi, idesc_kn,
+                             (i != 0) || (ks != 0));
+          tc::umma_commit(&sh->dv_done);
+        }
+        __syncwarp();
+      }
+      if (i + 1 < n) {
+        if (!wait(&sh->q_full[sn], parn, 50) || !wait(&sh->dv_done, par, 51)) break;
+        tc::tc_fence_after_sync();
+        issue_s(i + 1);
+      }
+      if (!wait(&sh->ds_full, par, 52)) break;
+      tc::tc_fence_after_sync();
+      {
+        const uint32_t q = tc::desc_lo(aQ + s * TILE, MN);
+        if (tc::elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < BKB / 16; ++ks)
+            tc::umma_bf16_lo<1>(tDP, ds_n + nstep(ks), hi, k_n + nstep(ks), hi, idesc_nn, ks != 0);
+          tc::umma_commit(&sh->dq_full);
+#pragma unroll
+          for (int ks = 0; ks < BQ / 16; ++ks)
+            tc::umma_bf16_lo<1>(tDK, ds_k + kstep(ks), hi, q + nstep(ks), hi, idesc_kn,
+                                (i != 0) || (ks != 0));
+          tc::umma_commit(&sh->q_empty[s]);
+          if (i + 1 == n) tc::umma_commit(&sh->fin);
+        }
+        __syncwarp();
+      }
+      if (i + 1 < n) {
+        if (!wait(&sh->do_full[sn], parn, 53) || !wait(&sh->dq_drained, par, 54)) break;
+        tc::tc_fence_after_sync();
+        issue_dp(i + 1);
+      }
+    }
+  } else {
+    // ------------------------------- loader ----------------------------------------------
+    auto load_tile = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col, int row) {
+#pragma unroll
+      for (int c = 0; c < HD / 64; ++c)
+        tc::tma_load_2d(dst + c * 128 * 128, map, bar, col + 64 * c, row);
+    };
+    if (tc::elect_one()) {
+      tc::mbar_expect_tx(&sh->kv_full, 2 * TILE);
+      load_tile(sK, &tm_qkv, &sh->kv_full, k_col, key0);
+      load_tile(sV, &tm_qkv, &sh->kv_full, v_col, key0);
+    }
+    __syncwarp();
+    for (int i = 0; i < n; ++i) {
+      const int s = i & 1;
+      const uint32_t par2 = ((uint32_t)(i >> 1) & 1u) ^ 1u;
+      const int row = b * p.seq + (kb + i) * BQ;
+      const size_t stat = ((size_t)b * p.heads + h) * p.seq + (size_t)(kb + i) * BQ;
+      if (!wait(&sh->q_empty[s], par2, 55)) break;
+      if (tc::elect_one()) {
+        tc::mbar_expect_tx(&sh->q_full[s], TILE + 2 * BQ * 4);
+        load_tile(sQ + s * TILE, &tm_qkv, &sh->q_full[s], q_col, row);
+        tc::bulk_load(sh->lse[s], p.lse2 + stat, BQ * 4, &sh->q_full[s]);
+        tc::bulk_load(sh->delta[s], p.delta + stat, BQ * 4, &sh->q_full[s]);
+      }
+      __syncwarp();
+      if (!wait(&sh->do_empty[s], par2, 56)) break;
+      if (tc::elect_one()) {
+        tc::mbar_expect_tx(&sh->do_full[s], TILE);
+        load_tile(sDO + s * TILE, &tm_do, &sh->do_full[s], q_col, row);
+      }
+      __syncwarp();
+    }
+    // Nothing may land after the CTA has left: the issuer has waited for every full barrier of
+    // the loads above unless a wait ran out.
+  }
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 12) {
+    tc::tc_fence_after_sync();
+    tc::tmem_dealloc(tmem, 512);
+  }
+}
+
 // delta[b, h, s] = sum_d dO * O   (one warp per (token, head), HD / 32 elements per lane)
 template <int HD>
 __global__ void __launch_bounds__(256)
@@ -988,8 +1377,9 @@ static int launch_fwd(const void* qkv, void* out, void* lse2, int batch, int seq
   return (int)cudaGetLastError();
 }
 
-// 0: float4 atomics, 1: TMA reduce-add from shared memory
-static int g_bwd_dq_variant = 1;
+// 0: float4 atomics, 1: TMA reduce-add from shared memory, 2: the software-pipelined kernel (which
+// reduces by TMA as well)
+static int g_bwd_dq_variant = 2;
 // 0: attention_fwd_kernel, 1: attention_fwd_pipelined_kernel
 static int g_fwd_variant = 1;
 
@@ -1050,9 +1440,14 @@ static int launch_bwd(const void* qkv, const void* out, const void* d_out, const
   CUtensorMap tm_qkv, tm_do, tm_dq;
   if (make_map(&tm_qkv, qkv, tokens, 3 * H, 64, 128)) return 1003;
   if (make_map(&tm_do, d_out, tokens, H, 64, 128)) return 1004;
+  // the pipelined kernel copies the row statistics with bulk copies
+  const bool pipelined =
+      g_bwd_dq_variant == 2 && !((uintptr_t)lse2 & 15) && !((uintptr_t)delta & 15);
   const bool tma_dq = g_bwd_dq_variant >= 1;
   if (tma_dq) {
-    if (((uintptr_t)dq_acc & 15) || make_map_f32(&tm_dq, dq_acc, tokens, H, 32, 128)) return 1007;
+    if (((uintptr_t)dq_acc & 15) ||
+        make_map_f32(&tm_dq, dq_acc, tokens, H, 32, pipelined ? 32 : 128))
+      return 1007;
   } else {
     tm_dq = tm_do;  // unused by the kernel
   }
@@ -1074,9 +1469,17 @@ static int launch_bwd(const void* qkv, const void* out, const void* d_out, const
   p.scale = scale;
   p.scale_log2 = scale * kLog2e;
   const int grid = batch * heads * (seq / BKB);
-  const int rc = tma_dq ? launch_bwd_kernel<HD, true>(tm_qkv, tm_do, tm_dq, p, grid, st)
-                        : launch_bwd_kernel<HD, false>(tm_qkv, tm_do, tm_dq, p, grid, st);
-  if (rc) return rc;
+  if (pipelined) {
+    if (!tc::ensure_dynamic_smem((const void*)attention_bwd_pipelined_kernel<HD>,
+                                 BwdPipe<HD>::SMEM))
+      return 1005;
+    attention_bwd_pipelined_kernel<HD><<<grid, kBwdPipeThreads, BwdPipe<HD>::SMEM, st>>>(
+        tm_qkv, tm_do, tm_dq, p);
+  } else {
+    const int rc = tma_dq ? launch_bwd_kernel<HD, true>(tm_qkv, tm_do, tm_dq, p, grid, st)
+                          : launch_bwd_kernel<HD, false>(tm_qkv, tm_do, tm_dq, p, grid, st);
+    if (rc) return rc;
+  }
   {
     const int col_blocks = (H / 4 + 255) / 256;
     long long rows = (tokens + 3) / 4;
@@ -1097,10 +1500,11 @@ static bool shape_ok(int batch, int seq, int heads, int head_dim) {
 extern "C" {
 
 // 0: dQ tiles are added to the fp32 accumulator with float4 atomics; 1: with TMA reductions
-// from a shared-memory staging tile.  Returns the previous value.
+// from a shared-memory staging tile; 2 (default): the software-pipelined kernel.  Returns the
+// previous value.
 int bcom_attention_set_bwd_dq_variant(int variant) {
   const int old = attn::g_bwd_dq_variant;
-  if (variant >= 0 && variant <= 1) attn::g_bwd_dq_variant = variant;
+  if (variant >= 0 && variant <= 2) attn::g_bwd_dq_variant = variant;
   return old;
 }
 

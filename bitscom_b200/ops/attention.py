@@ -19,9 +19,10 @@ _scratch: Dict[Tuple, torch.Tensor] = {}
 # forward kernels: "simple" alternates MMA and softmax inside a CTA; "pipelined" has an issuer
 # warp, double-buffered scores in TMEM and the output accumulated in TMEM
 _FWD_VARIANTS = {"simple": 0, "pipelined": 1}
-# how the backward kernel adds a dQ tile to the fp32 accumulator: float4 atomics from
-# registers, or TMA reductions from a shared-memory staging tile
-_BWD_DQ_VARIANTS = {"atomic": 0, "tma": 1}
+# backward kernels: MMA groups and softmax take turns and a dQ tile is added to the fp32
+# accumulator by float4 atomics from registers or by TMA reductions from a staging tile, or the
+# software-pipelined kernel (default; TMA reductions as well)
+_BWD_DQ_VARIANTS = {"atomic": 0, "tma": 1, "pipelined": 2}
 
 
 def _get():
@@ -64,7 +65,7 @@ def set_forward_variant(name: str) -> str:
 
 
 def set_backward_dq_variant(name: str) -> str:
-    """Select how dQ tiles are accumulated ("atomic" or "tma", also ``BITSCOM_ATTN_BWD_DQ``);
+    """Select the backward kernel ("atomic", "tma" or "pipelined", also ``BITSCOM_ATTN_BWD_DQ``);
     returns the name that was active before."""
     if name not in _BWD_DQ_VARIANTS:
         raise ValueError(f"unknown attention backward dQ variant {name!r}")
@@ -72,7 +73,7 @@ def set_backward_dq_variant(name: str) -> str:
     if lib is None:
         raise NativeError("attention kernel needs the bcom_llama library and a GPU")
     old = lib.bcom_attention_set_bwd_dq_variant(_BWD_DQ_VARIANTS[name])
-    return {0: "atomic", 1: "tma"}[old]
+    return {0: "atomic", 1: "tma", 2: "pipelined"}[old]
 
 
 def supported(seq: int, head_dim: int) -> bool:
