@@ -903,11 +903,13 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box {64, 1
 // for another one's whole step.  In the kernel above one thread issues the MMAs, everybody
 // waits for them, everybody does the element-wise part, and the next Q / dO tiles are requested
 // only after the last MMA: 13 k cycles per 128 x 128 block where the five products take 2.6 k.
-//   warps 0-7   softmax: P^T (bf16) goes back into tensor memory, over the S^T columns the warp
-//               has just read, and is the A operand of dV from there; dS^T goes to shared memory
-//   warps 8-11  dQ: tensor memory -> staging -> bulk reductions into the fp32 accumulator, each
+//   warps 0-15  softmax, 32 columns each: P^T (bf16) goes back into tensor memory, over the S^T
+//               columns the warp has just read, and is the A operand of dV from there; dS^T goes
+//               to shared memory.  (Eight warps of 64 columns: their two phases took 2.7-3.0 k of
+//               the 3.8-4.9 k cycles of a block.)
+//   warps 16-19 dQ: tensor memory -> staging -> bulk reductions into the fp32 accumulator, each
 //               warp its own 32 rows, in two halves of HD / 2 columns
-//   warp 12     issuer, warp 13 loader
+//   warp 20     issuer, warp 21 loader
 // Order on the tensor pipe: S_0 dP_0 | dV_0 S_1 dQ_0 dK_0 dP_1 | dV_1 S_2 dQ_1 dK_1 dP_2 | ...
 // so the exponentials of block i + 1 run under dQ_i dK_i dP_{i+1}, and dS_{i+1} under dV_{i+1}
 // S_{i+2}.  P^T in tensor memory leaves the shared memory for two Q and two dO tiles; dQ is
@@ -920,7 +922,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box {64, 1
 //   dO [s]              staging after dq_full(i), whose commit follows dV_i; loaded after do_empty
 //                       (the reductions have read the staging tile)
 // Measured (B2 S2048 H32 D128): 391 -> BWD_US us; (B8 S1024 H16 D64): 189 -> BWD64_US us.
-constexpr int kBwdPipeThreads = 14 * 32;
+constexpr int kBwdSoftmaxWarps = 16;
+constexpr int kBwdPipeThreads = (kBwdSoftmaxWarps + 6) * 32;
 
 struct BwdPipeShared {
   float lse[2][BQ], delta[2][BQ];
@@ -941,6 +944,7 @@ __global__ void __launch_bounds__(kBwdPipeThreads, 1)
 attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {64, 128}
                                const __grid_constant__ CUtensorMap tm_do,   // box {64, 128}
                                const __grid_constant__ CUtensorMap tm_dq,   // fp32, box {32, 32}
+                               const __grid_constant__ CUtensorMap tm_dkv,  // dqkv, box {64, 128}
                                const BwdParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int TILE = BwdPipe<HD>::TILE;
@@ -977,8 +981,8 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
     }
     tc::mbar_init(&sh->s_full, 1);
     tc::mbar_init(&sh->dp_full, 1);
-    tc::mbar_init(&sh->p_full, 8);
-    tc::mbar_init(&sh->ds_full, 8);
+    tc::mbar_init(&sh->p_full, kBwdSoftmaxWarps);
+    tc::mbar_init(&sh->ds_full, kBwdSoftmaxWarps);
     tc::mbar_init(&sh->dv_done, 1);
     tc::mbar_init(&sh->dq_full, 1);
     tc::mbar_init(&sh->dq_drained, 4);
@@ -986,7 +990,7 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
     sh->abort = 0;
     tc::fence_mbar_init();
   }
-  if (warp == 12) tc::tmem_alloc(&sh->tmem_base, 512);
+  if (warp == kBwdSoftmaxWarps + 4) tc::tmem_alloc(&sh->tmem_base, 512);
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
@@ -1011,44 +1015,41 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
     if (lane == 0) tc::mbar_arrive(bar);
   };
 
-  if (warp < 8) {
+  if (warp < kBwdSoftmaxWarps) {
     // ------------------------------- softmax ------------------------------------------
     const int row = ((warp & 3) << 5) | lane;  // key row
-    const int half = warp >> 2;                // query columns [64 half, 64 half + 64)
+    const int g = warp >> 2;                   // query columns [32 g, 32 g + 32)
     for (int i = 0; i < n; ++i) {
       const uint32_t par = (uint32_t)i & 1u, par2 = (uint32_t)(i >> 1) & 1u;
-      const float* lse = sh->lse[i & 1] + half * 64;
-      const float* delta = sh->delta[i & 1] + half * 64;
+      const float* lse = sh->lse[i & 1] + g * 32;
+      const float* delta = sh->delta[i & 1] + g * 32;
       if (!wait(&sh->q_full[i & 1], par2, 41) || !wait(&sh->s_full, par, 42)) break;
       tc::tc_fence_after_sync();
-      float pt[64];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      float pt[32];
+      {
         uint32_t r[32];
-        tc::tmem_ld_32x32(tS + lane_addr + half * 64 + c * 32, r);
+        tc::tmem_ld_32x32(tS + lane_addr + g * 32, r);
         tc::tmem_wait_ld();
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
-          const float4 l = *reinterpret_cast<const float4*>(lse + c * 32 + v * 4);
+          const float4 l = *reinterpret_cast<const float4*>(lse + v * 4);
           const float ls[4] = {l.x, l.y, l.z, l.w};
 #pragma unroll
           for (int u = 0; u < 4; ++u)
-            pt[c * 32 + v * 4 + u] =
-                ex2_fast(__uint_as_float(r[v * 4 + u]) * p.scale_log2 - ls[u]);
+            pt[v * 4 + u] = ex2_fast(__uint_as_float(r[v * 4 + u]) * p.scale_log2 - ls[u]);
         }
       }
       if (i == 0) {  // the block on the diagonal: query >= key
-        const int first = row - half * 64;  // columns before it are masked
+        const int first = row - g * 32;  // columns before it are masked
 #pragma unroll
-        for (int c = 0; c < 64; ++c)
+        for (int c = 0; c < 32; ++c)
           if (c < first) pt[c] = 0.0f;
       }
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      {
         uint32_t w[16];
 #pragma unroll
-        for (int v = 0; v < 16; ++v) w[v] = pack_bf16(pt[c * 32 + 2 * v], pt[c * 32 + 2 * v + 1]);
-        tc::tmem_st_32x16(tS + lane_addr + half * 64 + c * 16, w);
+        for (int v = 0; v < 16; ++v) w[v] = pack_bf16(pt[2 * v], pt[2 * v + 1]);
+        tc::tmem_st_32x16(tS + lane_addr + g * 32, w);
       }
       tc::tmem_wait_st();
       tc::tc_fence_before_sync();
@@ -1056,21 +1057,20 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
 
       if (!wait(&sh->dp_full, par, 43)) break;
       tc::tc_fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      {
         uint32_t r[32];
-        tc::tmem_ld_32x32(tDP + lane_addr + half * 64 + c * 32, r);
+        tc::tmem_ld_32x32(tDP + lane_addr + g * 32, r);
         tc::tmem_wait_ld();
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-          const float4 d0 = *reinterpret_cast<const float4*>(delta + c * 32 + v * 8);
-          const float4 d1 = *reinterpret_cast<const float4*>(delta + c * 32 + v * 8 + 4);
+          const float4 d0 = *reinterpret_cast<const float4*>(delta + v * 8);
+          const float4 d1 = *reinterpret_cast<const float4*>(delta + v * 8 + 4);
           const float dl[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
           float ds[8];
 #pragma unroll
           for (int u = 0; u < 8; ++u)
-            ds[u] = pt[c * 32 + v * 8 + u] * (__uint_as_float(r[v * 8 + u]) - dl[u]) * p.scale;
-          *reinterpret_cast<uint4*>(sDS + half * 128 * 128 + swz(row, c * 4 + v)) =
+            ds[u] = pt[v * 8 + u] * (__uint_as_float(r[v * 8 + u]) - dl[u]) * p.scale;
+          *reinterpret_cast<uint4*>(sDS + (g >> 1) * 128 * 128 + swz(row, (g & 1) * 4 + v)) =
               make_uint4(pack_bf16(ds[0], ds[1]), pack_bf16(ds[2], ds[3]),
                          pack_bf16(ds[4], ds[5]), pack_bf16(ds[6], ds[7]));
         }
@@ -1079,32 +1079,41 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
       tc::tc_fence_before_sync();    // dP^T has been read
       arrive(&sh->ds_full);
     }
-    // ---- dK, dV rows (thread t <-> key row t; the two halves split the columns) ----
+    // ---- dK, dV: through the K and V tiles, which are at rest, so that they leave as whole
+    // lines (16 bytes per lane and row straight to memory took about 4 us per CTA) ----
     if (wait(&sh->fin, 0, 44)) {
       tc::tc_fence_after_sync();
-      __nv_bfloat16* dk = p.dqkv + (size_t)(key0 + row) * 3 * H + k_col;
-      __nv_bfloat16* dv = p.dqkv + (size_t)(key0 + row) * 3 * H + v_col;
 #pragma unroll 1
-      for (int c = half * (HD / 64); c < (half + 1) * (HD / 64); ++c) {
-#pragma unroll 1
-        for (int t = 0; t < 2; ++t) {
-          uint32_t r[32];
-          tc::tmem_ld_32x32((t ? tDV : tDK) + lane_addr + c * 32, r);
-          tc::tmem_wait_ld();
-          uint4* dst = reinterpret_cast<uint4*>((t ? dv : dk) + c * 32);
+      for (int u = g; u < 2 * (HD / 32); u += 4) {
+        const int t = u / (HD / 32), c = u % (HD / 32);
+        uint32_t r[32];
+        tc::tmem_ld_32x32((t ? tDV : tDK) + lane_addr + c * 32, r);
+        tc::tmem_wait_ld();
+        uint8_t* dst = (t ? sV : sK) + (c >> 1) * 128 * 128;
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            dst[u] = make_uint4(
-                pack_bf16(__uint_as_float(r[u * 8 + 0]), __uint_as_float(r[u * 8 + 1])),
-                pack_bf16(__uint_as_float(r[u * 8 + 2]), __uint_as_float(r[u * 8 + 3])),
-                pack_bf16(__uint_as_float(r[u * 8 + 4]), __uint_as_float(r[u * 8 + 5])),
-                pack_bf16(__uint_as_float(r[u * 8 + 6]), __uint_as_float(r[u * 8 + 7])));
-        }
+        for (int v = 0; v < 4; ++v)
+          *reinterpret_cast<uint4*>(dst + swz(row, (c & 1) * 4 + v)) = make_uint4(
+              pack_bf16(__uint_as_float(r[v * 8 + 0]), __uint_as_float(r[v * 8 + 1])),
+              pack_bf16(__uint_as_float(r[v * 8 + 2]), __uint_as_float(r[v * 8 + 3])),
+              pack_bf16(__uint_as_float(r[v * 8 + 4]), __uint_as_float(r[v * 8 + 5])),
+              pack_bf16(__uint_as_float(r[v * 8 + 6]), __uint_as_float(r[v * 8 + 7])));
       }
+      tc::fence_proxy_async();
     }
-  } else if (warp < 12) {
+    // every softmax warp comes here, also after a wait that ran out
+    asm volatile("bar.sync 1, %0;" ::"n"(kBwdSoftmaxWarps * 32) : "memory");
+    if (tid == 0 && ok && !sh->abort) {
+#pragma unroll
+      for (int c = 0; c < HD / 64; ++c) {
+        tc::tma_store_2d(&tm_dkv, sK + c * 128 * 128, k_col + 64 * c, key0);
+        tc::tma_store_2d(&tm_dkv, sV + c * 128 * 128, v_col + 64 * c, key0);
+      }
+      tc::bulk_commit_group();
+      tc::bulk_wait_group0();
+    }
+  } else if (warp < kBwdSoftmaxWarps + 4) {
     // ------------------------------- dQ ------------------------------------------------
-    const int w = warp - 8;
+    const int w = warp - kBwdSoftmaxWarps;
     constexpr int SUB = HD / 64;  // 32-column sub-tiles per half
     for (int i = 0; i < n; ++i) {
       uint8_t* stage = sDO + (i & 1) * TILE + w * (SUB * 4096);
@@ -1144,7 +1153,7 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
     }
     if (lane == 0) tc::bulk_wait_group0();  // the reductions are performed before the CTA exits
     __syncwarp();
-  } else if (warp == 12) {
+  } else if (warp == kBwdSoftmaxWarps + 4) {
     // ------------------------------- issuer ---------------------------------------------
     constexpr uint32_t idesc_kk = tc::make_idesc_bf16(128, 128, false, false);  // both K-major
     constexpr uint32_t idesc_kn = tc::make_idesc_bf16(128, HD, false, true);    // B MN-major
@@ -1197,7 +1206,7 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
         if (tc::elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < BQ / 16; ++ks)
-            tc::umma_bf16_ta(tDV, tS + (ks >> 2) * 64 + (ks & 3) * 8, g + nstep(ks), hi, idesc_kn,
+            tc::umma_bf16_ta(tDV, tS + (ks >> 1) * 32 + (ks & 1) * 8, g + nstep(ks), hi, idesc_kn,
                              (i != 0) || (ks != 0));
           tc::umma_commit(&sh->dv_done);
         }
@@ -1270,38 +1279,65 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
   }
   tc::tc_fence_before_sync();
   __syncthreads();
-  if (warp == 12) {
+  if (warp == kBwdSoftmaxWarps + 4) {
     tc::tc_fence_after_sync();
     tc::tmem_dealloc(tmem, 512);
   }
 }
 
-// delta[b, h, s] = sum_d dO * O   (one warp per (token, head), HD / 32 elements per lane)
+// delta[b, h, s] = sum_d dO * O.  HD / 8 adjacent lanes share a (token, head) and load 16 bytes
+// each of both tensors; two of them per thread are in flight.  (One warp per pair with 4 or 8
+// bytes per lane: 25 us for 67 MB at B2 S2048 H32 D128, 24 us for 34 MB at B8 S1024 H16 D64.)
 template <int HD>
 __global__ void __launch_bounds__(256)
 attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                       float* __restrict__ delta, int batch, int seq, int heads) {
-  const int lane = threadIdx.x & 31;
-  const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long total = (long long)batch * seq * heads;
-  if (warp_id >= total) return;
-  const int h = (int)(warp_id % heads);
-  const long long tok = warp_id / heads;
-  constexpr int PAIRS = HD / 64;  // bf16 pairs per lane
-  const size_t off = (size_t)tok * heads * HD + (size_t)h * HD + lane * (2 * PAIRS);
-  const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(o + off);
-  const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(d_o + off);
-  float s = 0.0f;
+                       float* __restrict__ delta, int batch, int seq, int heads, bool aligned) {
+  constexpr int LANES = HD / 8;
+  const long long total = (long long)batch * seq * heads;  // (token, head) pairs, head fastest
+  const int sub = threadIdx.x % LANES;
+  const long long stride = (long long)gridDim.x * (blockDim.x / LANES);
+  const long long first = (long long)blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
+  auto dot = [](const uint4& x, const uint4& y) {
+    const uint32_t a[4] = {x.x, x.y, x.z, x.w}, g[4] = {y.x, y.y, y.z, y.w};
+    float s = 0.0f;
 #pragma unroll
-  for (int i = 0; i < PAIRS; ++i) {
-    const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(g2[i]);
-    s += x.x * y.x + x.y * y.y;
-  }
+    for (int i = 0; i < 4; ++i)
+      s += __uint_as_float(a[i] << 16) * __uint_as_float(g[i] << 16) +
+           __uint_as_float(a[i] & 0xffff0000u) * __uint_as_float(g[i] & 0xffff0000u);
+    return s;
+  };
+  auto load = [&](const __nv_bfloat16* p) {
+    if (aligned) return __ldg(reinterpret_cast<const uint4*>(p));
+    uint32_t w[4];
+    const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
 #pragma unroll
-  for (int w = 16; w > 0; w >>= 1) s += __shfl_xor_sync(0xffffffffu, s, w);
-  if (lane == 0) {
-    const int b = (int)(tok / seq), sp = (int)(tok % seq);
-    delta[((size_t)b * heads + h) * seq + sp] = s;
+    for (int i = 0; i < 4; ++i) w[i] = (uint32_t)q[2 * i] | ((uint32_t)q[2 * i + 1] << 16);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  };
+  auto finish = [&](float s, long long pair) {
+#pragma unroll
+    for (int w = LANES / 2; w > 0; w >>= 1) s += __shfl_xor_sync(0xffffffffu, s, w);
+    if (sub == 0 && pair < total) {
+      const int h = (int)(pair % heads);
+      const long long tok = pair / heads;
+      const int b = (int)(tok / seq), sp = (int)(tok - (long long)b * seq);
+      delta[((size_t)b * heads + h) * seq + sp] = s;
+    }
+  };
+  // the loop bound is uniform over a warp: its lanes' pairs are adjacent, the shuffles need all
+  for (long long p0 = first; p0 - threadIdx.x / LANES < total; p0 += 2 * stride) {
+    const long long p1 = p0 + stride;
+    uint4 a0 = make_uint4(0, 0, 0, 0), g0 = a0, a1 = a0, g1 = a0;
+    if (p0 < total) {
+      a0 = load(o + p0 * HD + sub * 8);
+      g0 = load(d_o + p0 * HD + sub * 8);
+    }
+    if (p1 < total) {
+      a1 = load(o + p1 * HD + sub * 8);
+      g1 = load(d_o + p1 * HD + sub * 8);
+    }
+    finish(dot(a0, g0), p0);
+    finish(dot(a1, g1), p1);
   }
 }
 
@@ -1452,11 +1488,13 @@ static int launch_bwd(const void* qkv, const void* out, const void* d_out, const
     tm_dq = tm_do;  // unused by the kernel
   }
   {
-    const long long warps = tokens * heads;
-    const int grid = (int)((warps * 32 + 255) / 256);
+    const long long per_cta = 2 * 256 / (HD / 8);
+    const long long want = (tokens * heads + per_cta - 1) / per_cta;
+    const int grid = (int)(want < 148 * 8 ? want : 148 * 8);
     attention_delta_kernel<HD><<<grid, 256, 0, st>>>((const __nv_bfloat16*)out,
                                                      (const __nv_bfloat16*)d_out, delta, batch,
-                                                     seq, heads);
+                                                     seq, heads,
+                                                     (((uintptr_t)out | (uintptr_t)d_out) & 15) == 0);
   }
   BwdParams p;
   p.dqkv = (__nv_bfloat16*)dqkv;
@@ -1473,8 +1511,10 @@ static int launch_bwd(const void* qkv, const void* out, const void* d_out, const
     if (!tc::ensure_dynamic_smem((const void*)attention_bwd_pipelined_kernel<HD>,
                                  BwdPipe<HD>::SMEM))
       return 1005;
+    CUtensorMap tm_dkv;
+    if (make_map(&tm_dkv, dqkv, tokens, 3 * H, 64, 128)) return 1008;
     attention_bwd_pipelined_kernel<HD><<<grid, kBwdPipeThreads, BwdPipe<HD>::SMEM, st>>>(
-        tm_qkv, tm_do, tm_dq, p);
+        tm_qkv, tm_do, tm_dq, tm_dkv, p);
   } else {
     const int rc = tma_dq ? launch_bwd_kernel<HD, true>(tm_qkv, tm_do, tm_dq, p, grid, st)
                           : launch_bwd_kernel<HD, false>(tm_qkv, tm_do, tm_dq, p, grid, st);
