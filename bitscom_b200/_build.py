@@ -35,7 +35,8 @@ LIBRARIES: Dict[str, dict] = {
                   "deps": ["codec.cuh", "symm.h"], "flags": []},
     "bcom_cpu": {"sources": ["cpu_codec.cc"], "deps": [], "flags": [], "host_only": True},
     "bcom_llama": {"sources": ["gemm_tcgen05.cu", "attention_tcgen05.cu", "elementwise.cu"],
-                   "deps": ["tc_common.cuh", "gemm_epilogue.cuh", "gemm_schedule.cuh", "no_alloc.h"],
+                   "deps": ["tc_common.cuh", "gemm_epilogue.cuh", "gemm_schedule.cuh",
+                            "attention_schedule.cuh", "no_alloc.h"],
                    "flags": []},
     # CTA-pair GEMM (opt-in variant): a library of its own, so that it can be left out of a
     # deployment without touching the default kernels

@@ -33,6 +33,7 @@
 #include <cstdio>
 #include <mutex>
 
+#include "attention_schedule.cuh"
 #include "tc_common.cuh"
 
 namespace attn {
@@ -917,18 +918,27 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv,   // box {64, 1
 // Why each buffer may be written when it is:
 //   S (and P over it)   S_{i+1} is issued after dV_i has completed (dv_done)
 //   dP (and dQ over it) dQ_i after ds_full(i) (dP_i read), dP_{i+1} after dq_drained(i)
-//   dS                  written after dp_full(i+1), whose commit follows dQ_i and dK_i
+//   dS                  written after dp_full(i+1), whose commit follows dQ_i and dK_i; it also
+//                       stages dK of an item, the next item's first dS waits for st_done
+//   dV, dK              the next item's first dV waits for acc_drained
 //   Q, lse, delta [s]   loaded after q_empty (dK_i complete, hence ds_full(i))
 //   dO [s]              staging after dq_full(i), whose commit follows dV_i; loaded after do_empty
 //                       (the reductions have read the staging tile)
-// Measured (B2 S2048 H32 D128): 391 -> BWD_US us; (B8 S1024 H16 D64): 189 -> BWD64_US us.
+// One persistent CTA per SM walks (key block, head) items, most query blocks first and back and
+// forth over the CTAs (attention_schedule.cuh), so that start-up, first loads and the write-out
+// of an item run under its neighbours: as one CTA per item they were 8 of 32 us (head_dim 128).
+// What bounds it now at head_dim 128 is shared memory: 288 KiB of operands, 64 KiB loads, 32 KiB
+// dS and twice 64 KiB of dQ staging per block are 4.1 k cycles at 128 bytes per cycle.
 constexpr int kBwdSoftmaxWarps = 16;
 constexpr int kBwdPipeThreads = (kBwdSoftmaxWarps + 6) * 32;
 
 struct BwdPipeShared {
   float lse[2][BQ], delta[2][BQ];
-  uint64_t kv_full, q_full[2], do_full[2], q_empty[2], do_empty[2];
-  uint64_t s_full, dp_full, p_full, ds_full, dv_done, dq_full, dq_drained, fin;
+  // per block (phase = running block number), two-stage rings for Q and dO
+  uint64_t q_full[2], do_full[2], q_empty[2], do_empty[2];
+  uint64_t s_full, dp_full, p_full, ds_full, dv_done, dq_full, dq_drained;
+  // per work item
+  uint64_t k_full, v_full, fin, acc_drained, staged, st_done;
   uint32_t tmem_base;
   volatile int abort;
 };
@@ -960,19 +970,9 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
     if (tid == 0) record_fail(40);
     return;
   }
-  const int kblocks = p.seq / BKB;
-  // key blocks with the most query blocks first, over all heads: the last ones to start are short
-  const int heads = p.batch * p.heads;
-  const int kb = (int)blockIdx.x / heads;
-  const int bh = (int)blockIdx.x - kb * heads;
-  const int h = bh % p.heads, b = bh / p.heads;
   const int H = p.heads * HD;
-  const int key0 = b * p.seq + kb * BKB;
-  const int q_col = h * HD, k_col = H + h * HD, v_col = 2 * H + h * HD;
-  const int n = kblocks - kb;  // query blocks kb .. kblocks-1 (BQ == BKB)
 
   if (tid == 0) {
-    tc::mbar_init(&sh->kv_full, 1);
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&sh->q_full[i], 1);
       tc::mbar_init(&sh->do_full[i], 1);
@@ -986,7 +986,12 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
     tc::mbar_init(&sh->dv_done, 1);
     tc::mbar_init(&sh->dq_full, 1);
     tc::mbar_init(&sh->dq_drained, 4);
+    tc::mbar_init(&sh->k_full, 1);
+    tc::mbar_init(&sh->v_full, 1);
     tc::mbar_init(&sh->fin, 1);
+    tc::mbar_init(&sh->acc_drained, kBwdSoftmaxWarps);
+    tc::mbar_init(&sh->staged, kBwdSoftmaxWarps);
+    tc::mbar_init(&sh->st_done, 1);
     sh->abort = 0;
     tc::fence_mbar_init();
   }
@@ -1001,7 +1006,7 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
   bool ok = true;
   // every lane of a warp waits; the verdict is uniform
   auto wait = [&](uint64_t* bar, uint32_t parity, unsigned code) {
-    if (ok && !tc::mbar_wait_warp(bar, parity, kBudgetNs)) {
+    if (ok && !tc::mbar_wait_warp(bar, parity & 1u, kBudgetNs)) {
       ok = false;
       if (lane == 0) {
         sh->abort = 1;
@@ -1015,73 +1020,95 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
     if (lane == 0) tc::mbar_arrive(bar);
   };
 
+  // Work item j of this CTA.  `it` is the running block number of the CTA (the phase of the
+  // per-block barriers), every role counts it for itself.
+  struct Item {
+    int kb, b, h, n, key0;
+  };
+  const int kblocks = p.seq / BKB;
+  auto item = [&](int j, Item& w) {
+    const int t = attn_sched::item_index((int)blockIdx.x, (int)gridDim.x, j);
+    if (t >= kblocks * p.batch * p.heads) return false;
+    w.kb = t / (p.batch * p.heads);
+    const int bh = t - w.kb * p.batch * p.heads;
+    w.h = bh % p.heads;
+    w.b = bh / p.heads;
+    w.n = kblocks - w.kb;  // query blocks kb .. kblocks-1 (BQ == BKB)
+    w.key0 = w.b * p.seq + w.kb * BKB;
+    return true;
+  };
+  Item w;
+
   if (warp < kBwdSoftmaxWarps) {
     // ------------------------------- softmax ------------------------------------------
     const int row = ((warp & 3) << 5) | lane;  // key row
     const int g = warp >> 2;                   // query columns [32 g, 32 g + 32)
-    for (int i = 0; i < n; ++i) {
-      const uint32_t par = (uint32_t)i & 1u, par2 = (uint32_t)(i >> 1) & 1u;
-      const float* lse = sh->lse[i & 1] + g * 32;
-      const float* delta = sh->delta[i & 1] + g * 32;
-      if (!wait(&sh->q_full[i & 1], par2, 41) || !wait(&sh->s_full, par, 42)) break;
-      tc::tc_fence_after_sync();
-      float pt[32];
-      {
-        uint32_t r[32];
-        tc::tmem_ld_32x32(tS + lane_addr + g * 32, r);
-        tc::tmem_wait_ld();
+    uint32_t it = 0;
+    for (int j = 0; ok && item(j, w); ++j) {
+      for (int i = 0; i < w.n; ++i, ++it) {
+        const float* lse = sh->lse[it & 1] + g * 32;
+        const float* delta = sh->delta[it & 1] + g * 32;
+        if (!wait(&sh->q_full[it & 1], it >> 1, 41) || !wait(&sh->s_full, it, 42)) break;
+        tc::tc_fence_after_sync();
+        float pt[32];
+        {
+          uint32_t r[32];
+          tc::tmem_ld_32x32(tS + lane_addr + g * 32, r);
+          tc::tmem_wait_ld();
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          const float4 l = *reinterpret_cast<const float4*>(lse + v * 4);
-          const float ls[4] = {l.x, l.y, l.z, l.w};
+          for (int v = 0; v < 8; ++v) {
+            const float4 l = *reinterpret_cast<const float4*>(lse + v * 4);
+            const float ls[4] = {l.x, l.y, l.z, l.w};
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            pt[v * 4 + u] = ex2_fast(__uint_as_float(r[v * 4 + u]) * p.scale_log2 - ls[u]);
+            for (int u = 0; u < 4; ++u)
+              pt[v * 4 + u] = ex2_fast(__uint_as_float(r[v * 4 + u]) * p.scale_log2 - ls[u]);
+          }
         }
-      }
-      if (i == 0) {  // the block on the diagonal: query >= key
-        const int first = row - g * 32;  // columns before it are masked
+        if (i == 0) {  // the block on the diagonal: query >= key
+          const int first = row - g * 32;  // columns before it are masked
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
-          if (c < first) pt[c] = 0.0f;
-      }
-      {
-        uint32_t w[16];
+          for (int c = 0; c < 32; ++c)
+            if (c < first) pt[c] = 0.0f;
+        }
+        {
+          uint32_t pk[16];
 #pragma unroll
-        for (int v = 0; v < 16; ++v) w[v] = pack_bf16(pt[2 * v], pt[2 * v + 1]);
-        tc::tmem_st_32x16(tS + lane_addr + g * 32, w);
-      }
-      tc::tmem_wait_st();
-      tc::tc_fence_before_sync();
-      arrive(&sh->p_full);
+          for (int v = 0; v < 16; ++v) pk[v] = pack_bf16(pt[2 * v], pt[2 * v + 1]);
+          tc::tmem_st_32x16(tS + lane_addr + g * 32, pk);
+        }
+        tc::tmem_wait_st();
+        tc::tc_fence_before_sync();
+        arrive(&sh->p_full);
 
-      if (!wait(&sh->dp_full, par, 43)) break;
-      tc::tc_fence_after_sync();
-      {
-        uint32_t r[32];
-        tc::tmem_ld_32x32(tDP + lane_addr + g * 32, r);
-        tc::tmem_wait_ld();
+        if (!wait(&sh->dp_full, it, 43)) break;
+        // the dS tile staged the previous item's dK
+        if (i == 0 && j > 0 && !wait(&sh->st_done, (uint32_t)j - 1, 57)) break;
+        tc::tc_fence_after_sync();
+        {
+          uint32_t r[32];
+          tc::tmem_ld_32x32(tDP + lane_addr + g * 32, r);
+          tc::tmem_wait_ld();
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const float4 d0 = *reinterpret_cast<const float4*>(delta + v * 8);
-          const float4 d1 = *reinterpret_cast<const float4*>(delta + v * 8 + 4);
-          const float dl[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-          float ds[8];
+          for (int v = 0; v < 4; ++v) {
+            const float4 d0 = *reinterpret_cast<const float4*>(delta + v * 8);
+            const float4 d1 = *reinterpret_cast<const float4*>(delta + v * 8 + 4);
+            const float dl[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+            float ds[8];
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
-            ds[u] = pt[v * 8 + u] * (__uint_as_float(r[v * 8 + u]) - dl[u]) * p.scale;
-          *reinterpret_cast<uint4*>(sDS + (g >> 1) * 128 * 128 + swz(row, (g & 1) * 4 + v)) =
-              make_uint4(pack_bf16(ds[0], ds[1]), pack_bf16(ds[2], ds[3]),
-                         pack_bf16(ds[4], ds[5]), pack_bf16(ds[6], ds[7]));
+            for (int u = 0; u < 8; ++u)
+              ds[u] = pt[v * 8 + u] * (__uint_as_float(r[v * 8 + u]) - dl[u]) * p.scale;
+            *reinterpret_cast<uint4*>(sDS + (g >> 1) * 128 * 128 + swz(row, (g & 1) * 4 + v)) =
+                make_uint4(pack_bf16(ds[0], ds[1]), pack_bf16(ds[2], ds[3]),
+                           pack_bf16(ds[4], ds[5]), pack_bf16(ds[6], ds[7]));
+          }
         }
+        tc::fence_proxy_async();       // dS^T is visible to the MMA
+        tc::tc_fence_before_sync();    // dP^T has been read
+        arrive(&sh->ds_full);
       }
-      tc::fence_proxy_async();       // dS^T is visible to the MMA
-      tc::tc_fence_before_sync();    // dP^T has been read
-      arrive(&sh->ds_full);
-    }
-    // ---- dK, dV: through the K and V tiles, which are at rest, so that they leave as whole
-    // lines (16 bytes per lane and row straight to memory took about 4 us per CTA) ----
-    if (wait(&sh->fin, 0, 44)) {
+      // ---- dK, dV: through the dS and V tiles, which are at rest, so that they leave as whole
+      // lines while the next item's K and Q arrive ----
+      if (!wait(&sh->fin, (uint32_t)j, 44)) break;
       tc::tc_fence_after_sync();
 #pragma unroll 1
       for (int u = g; u < 2 * (HD / 32); u += 4) {
@@ -1089,7 +1116,7 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
         uint32_t r[32];
         tc::tmem_ld_32x32((t ? tDV : tDK) + lane_addr + c * 32, r);
         tc::tmem_wait_ld();
-        uint8_t* dst = (t ? sV : sK) + (c >> 1) * 128 * 128;
+        uint8_t* dst = (t ? sV : sDS) + (c >> 1) * 128 * 128;
 #pragma unroll
         for (int v = 0; v < 4; ++v)
           *reinterpret_cast<uint4*>(dst + swz(row, (c & 1) * 4 + v)) = make_uint4(
@@ -1099,57 +1126,70 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
               pack_bf16(__uint_as_float(r[v * 8 + 6]), __uint_as_float(r[v * 8 + 7])));
       }
       tc::fence_proxy_async();
-    }
-    // every softmax warp comes here, also after a wait that ran out
-    asm volatile("bar.sync 1, %0;" ::"n"(kBwdSoftmaxWarps * 32) : "memory");
-    if (tid == 0 && ok && !sh->abort) {
+      tc::tc_fence_before_sync();
+      arrive(&sh->acc_drained);
+      arrive(&sh->staged);
+      if (warp == 0) {
+        if (!wait(&sh->staged, (uint32_t)j, 58)) break;
+        if (lane == 0) {
+          const int k_col = H + w.h * HD, v_col = 2 * H + w.h * HD;
 #pragma unroll
-      for (int c = 0; c < HD / 64; ++c) {
-        tc::tma_store_2d(&tm_dkv, sK + c * 128 * 128, k_col + 64 * c, key0);
-        tc::tma_store_2d(&tm_dkv, sV + c * 128 * 128, v_col + 64 * c, key0);
+          for (int c = 0; c < HD / 64; ++c) {
+            tc::tma_store_2d(&tm_dkv, sDS + c * 128 * 128, k_col + 64 * c, w.key0);
+            tc::tma_store_2d(&tm_dkv, sV + c * 128 * 128, v_col + 64 * c, w.key0);
+          }
+          tc::bulk_commit_group();
+          tc::bulk_wait_group_read0();  // both tiles may be written again
+          tc::mbar_arrive(&sh->st_done);
+        }
+        __syncwarp();
       }
-      tc::bulk_commit_group();
-      tc::bulk_wait_group0();
     }
+    if (tid == 0) tc::bulk_wait_group0();
+    __syncwarp();
   } else if (warp < kBwdSoftmaxWarps + 4) {
     // ------------------------------- dQ ------------------------------------------------
-    const int w = warp - kBwdSoftmaxWarps;
+    const int dw = warp - kBwdSoftmaxWarps;
     constexpr int SUB = HD / 64;  // 32-column sub-tiles per half
-    for (int i = 0; i < n; ++i) {
-      uint8_t* stage = sDO + (i & 1) * TILE + w * (SUB * 4096);
-      const int qrow = b * p.seq + (kb + i) * BQ + w * 32;
-      if (!wait(&sh->dq_full, (uint32_t)i & 1u, 45)) break;
-      tc::tc_fence_after_sync();
+    uint32_t it = 0;
+    for (int j = 0; ok && item(j, w); ++j) {
+      const int q_col = w.h * HD;
+      for (int i = 0; i < w.n; ++i, ++it) {
+        uint8_t* stage = sDO + (it & 1) * TILE + dw * (SUB * 4096);
+        const int qrow = w.b * p.seq + (w.kb + i) * BQ + dw * 32;
+        if (!wait(&sh->dq_full, it, 45)) break;
+        tc::tc_fence_after_sync();
 #pragma unroll 1
-      for (int hf = 0; hf < 2; ++hf) {
-        uint32_t r[SUB][32];
-#pragma unroll
-        for (int c = 0; c < SUB; ++c)
-          tc::tmem_ld_32x32(tDP + lane_addr + hf * (HD / 2) + c * 32, r[c]);
-        tc::tmem_wait_ld();
-        if (hf == 1) {
-          tc::tc_fence_before_sync();
-          arrive(&sh->dq_drained);
-          if (lane == 0) tc::bulk_wait_group_read0();  // the first half has left the staging tile
-          __syncwarp();
-        }
-#pragma unroll
-        for (int c = 0; c < SUB; ++c)
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            *reinterpret_cast<uint4*>(stage + c * 4096 + swz(lane, u)) =
-                make_uint4(r[c][u * 4], r[c][u * 4 + 1], r[c][u * 4 + 2], r[c][u * 4 + 3]);
-        tc::fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) {
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t r[SUB][32];
 #pragma unroll
           for (int c = 0; c < SUB; ++c)
-            tc::tma_reduce_add_2d(&tm_dq, stage + c * 4096, q_col + hf * (HD / 2) + c * 32, qrow);
-          tc::bulk_commit_group();
+            tc::tmem_ld_32x32(tDP + lane_addr + hf * (HD / 2) + c * 32, r[c]);
+          tc::tmem_wait_ld();
+          if (hf == 1) {
+            tc::tc_fence_before_sync();
+            arrive(&sh->dq_drained);
+            if (lane == 0) tc::bulk_wait_group_read0();  // the first half has left the tile
+            __syncwarp();
+          }
+#pragma unroll
+          for (int c = 0; c < SUB; ++c)
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              *reinterpret_cast<uint4*>(stage + c * 4096 + swz(lane, u)) =
+                  make_uint4(r[c][u * 4], r[c][u * 4 + 1], r[c][u * 4 + 2], r[c][u * 4 + 3]);
+          tc::fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+#pragma unroll
+            for (int c = 0; c < SUB; ++c)
+              tc::tma_reduce_add_2d(&tm_dq, stage + c * 4096, q_col + hf * (HD / 2) + c * 32, qrow);
+            tc::bulk_commit_group();
+          }
         }
+        if (lane == 0) tc::bulk_wait_group_read0();
+        arrive(&sh->do_empty[it & 1]);
       }
-      if (lane == 0) tc::bulk_wait_group_read0();
-      arrive(&sh->do_empty[i & 1]);
     }
     if (lane == 0) tc::bulk_wait_group0();  // the reductions are performed before the CTA exits
     __syncwarp();
@@ -1167,8 +1207,12 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
     // k-step ks of a K-major operand (64-column chunks 16 KiB apart) and of an MN-major one
     auto kstep = [](int ks) { return (uint32_t)((ks >> 2) * (MN >> 4) + (ks & 3) * 2); };
     auto nstep = [](int ks) { return (uint32_t)(ks * (16 * 128 >> 4)); };
-    auto issue_s = [&](int i) {
-      const uint32_t q = tc::desc_lo(aQ + (i & 1) * TILE, 16);
+    // S of block t: its Q has landed and dV of the block before has read the P over it
+    auto issue_s = [&](uint32_t t) {
+      if (!wait(&sh->q_full[t & 1], t >> 1, 50)) return;
+      if (t > 0 && !wait(&sh->dv_done, t - 1, 51)) return;
+      tc::tc_fence_after_sync();
+      const uint32_t q = tc::desc_lo(aQ + (t & 1) * TILE, 16);
       if (tc::elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks)
@@ -1177,68 +1221,62 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
       }
       __syncwarp();
     };
-    auto issue_dp = [&](int i) {
-      const uint32_t g = tc::desc_lo(aDO + (i & 1) * TILE, 16);
+    // dP of block t: its dO has landed and dQ of the block before has been drained
+    auto issue_dp = [&](uint32_t t) {
+      if (!wait(&sh->do_full[t & 1], t >> 1, 53)) return;
+      if (t > 0 && !wait(&sh->dq_drained, t - 1, 54)) return;
+      tc::tc_fence_after_sync();
+      const uint32_t gd = tc::desc_lo(aDO + (t & 1) * TILE, 16);
       if (tc::elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks)
-          tc::umma_bf16_lo<1>(tDP, v_k + kstep(ks), hi, g + kstep(ks), hi, idesc_kk, ks != 0);
+          tc::umma_bf16_lo<1>(tDP, v_k + kstep(ks), hi, gd + kstep(ks), hi, idesc_kk, ks != 0);
         tc::umma_commit(&sh->dp_full);
       }
       __syncwarp();
     };
-    if (wait(&sh->kv_full, 0, 46) && wait(&sh->q_full[0], 0, 47)) {
-      tc::tc_fence_after_sync();
-      issue_s(0);
-      if (wait(&sh->do_full[0], 0, 48)) {
+    uint32_t it = 0;
+    for (int j = 0; ok && item(j, w); ++j) {
+      if (wait(&sh->k_full, (uint32_t)j, 46)) issue_s(it);
+      if (wait(&sh->v_full, (uint32_t)j, 47)) issue_dp(it);
+      for (int i = 0; i < w.n && ok; ++i, ++it) {
+        const int s = it & 1;
+        if (!wait(&sh->p_full, it, 49)) break;
+        // dV and dK of the item before have been read
+        if (i == 0 && j > 0 && !wait(&sh->acc_drained, (uint32_t)j - 1, 48)) break;
         tc::tc_fence_after_sync();
-        issue_dp(0);
-      }
-    }
-    for (int i = 0; i < n && ok; ++i) {
-      const uint32_t par = (uint32_t)i & 1u;
-      const int s = i & 1, sn = (i + 1) & 1;
-      const uint32_t parn = (uint32_t)((i + 1) >> 1) & 1u;
-      if (!wait(&sh->p_full, par, 49)) break;
-      tc::tc_fence_after_sync();
-      {
-        const uint32_t g = tc::desc_lo(aDO + s * TILE, MN);
-        if (tc::elect_one()) {
+        {
+          const uint32_t gd = tc::desc_lo(aDO + s * TILE, MN);
+          if (tc::elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < BQ / 16; ++ks)
-            tc::umma_bf16_ta(tDV, tS + (ks >> 1) * 32 + (ks & 1) * 8, g + nstep(ks), hi, idesc_kn,
-                             (i != 0) || (ks != 0));
-          tc::umma_commit(&sh->dv_done);
+            for (int ks = 0; ks < BQ / 16; ++ks)
+              tc::umma_bf16_ta(tDV, tS + (ks >> 1) * 32 + (ks & 1) * 8, gd + nstep(ks), hi,
+                               idesc_kn, (i != 0) || (ks != 0));
+            tc::umma_commit(&sh->dv_done);
+          }
+          __syncwarp();
         }
-        __syncwarp();
-      }
-      if (i + 1 < n) {
-        if (!wait(&sh->q_full[sn], parn, 50) || !wait(&sh->dv_done, par, 51)) break;
+        if (i + 1 < w.n) issue_s(it + 1);
+        if (!wait(&sh->ds_full, it, 52)) break;
         tc::tc_fence_after_sync();
-        issue_s(i + 1);
-      }
-      if (!wait(&sh->ds_full, par, 52)) break;
-      tc::tc_fence_after_sync();
-      {
-        const uint32_t q = tc::desc_lo(aQ + s * TILE, MN);
-        if (tc::elect_one()) {
+        {
+          const uint32_t q = tc::desc_lo(aQ + s * TILE, MN);
+          if (tc::elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < BKB / 16; ++ks)
-            tc::umma_bf16_lo<1>(tDP, ds_n + nstep(ks), hi, k_n + nstep(ks), hi, idesc_nn, ks != 0);
-          tc::umma_commit(&sh->dq_full);
+            for (int ks = 0; ks < BKB / 16; ++ks)
+              tc::umma_bf16_lo<1>(tDP, ds_n + nstep(ks), hi, k_n + nstep(ks), hi, idesc_nn,
+                                  ks != 0);
+            tc::umma_commit(&sh->dq_full);
 #pragma unroll
-          for (int ks = 0; ks < BQ / 16; ++ks)
-            tc::umma_bf16_lo<1>(tDK, ds_k + kstep(ks), hi, q + nstep(ks), hi, idesc_kn,
-                                (i != 0) || (ks != 0));
-          tc::umma_commit(&sh->q_empty[s]);
-          if (i + 1 == n) tc::umma_commit(&sh->fin);
+            for (int ks = 0; ks < BQ / 16; ++ks)
+              tc::umma_bf16_lo<1>(tDK, ds_k + kstep(ks), hi, q + nstep(ks), hi, idesc_kn,
+                                  (i != 0) || (ks != 0));
+            tc::umma_commit(&sh->q_empty[s]);
+            if (i + 1 == w.n) tc::umma_commit(&sh->fin);
+          }
+          __syncwarp();
         }
-        __syncwarp();
-      }
-      if (i + 1 < n) {
-        if (!wait(&sh->do_full[sn], parn, 53) || !wait(&sh->dq_drained, par, 54)) break;
-        tc::tc_fence_after_sync();
-        issue_dp(i + 1);
+        if (i + 1 < w.n) issue_dp(it + 1);
       }
     }
   } else {
@@ -1248,31 +1286,43 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
       for (int c = 0; c < HD / 64; ++c)
         tc::tma_load_2d(dst + c * 128 * 128, map, bar, col + 64 * c, row);
     };
-    if (tc::elect_one()) {
-      tc::mbar_expect_tx(&sh->kv_full, 2 * TILE);
-      load_tile(sK, &tm_qkv, &sh->kv_full, k_col, key0);
-      load_tile(sV, &tm_qkv, &sh->kv_full, v_col, key0);
-    }
-    __syncwarp();
-    for (int i = 0; i < n; ++i) {
-      const int s = i & 1;
-      const uint32_t par2 = ((uint32_t)(i >> 1) & 1u) ^ 1u;
-      const int row = b * p.seq + (kb + i) * BQ;
-      const size_t stat = ((size_t)b * p.heads + h) * p.seq + (size_t)(kb + i) * BQ;
-      if (!wait(&sh->q_empty[s], par2, 55)) break;
-      if (tc::elect_one()) {
-        tc::mbar_expect_tx(&sh->q_full[s], TILE + 2 * BQ * 4);
-        load_tile(sQ + s * TILE, &tm_qkv, &sh->q_full[s], q_col, row);
-        tc::bulk_load(sh->lse[s], p.lse2 + stat, BQ * 4, &sh->q_full[s]);
-        tc::bulk_load(sh->delta[s], p.delta + stat, BQ * 4, &sh->q_full[s]);
+    uint32_t it = 0;
+    for (int j = 0; ok && item(j, w); ++j) {
+      for (int i = 0; i < w.n; ++i, ++it) {
+        const int s = it & 1;
+        const uint32_t used = (it >> 1) + 1;  // parity of the phase before this one
+        const int row = w.b * p.seq + (w.kb + i) * BQ;
+        const size_t stat = ((size_t)w.b * p.heads + w.h) * p.seq + (size_t)(w.kb + i) * BQ;
+        if (!wait(&sh->q_empty[s], used, 55)) break;
+        if (tc::elect_one()) {
+          tc::mbar_expect_tx(&sh->q_full[s], TILE + 2 * BQ * 4);
+          load_tile(sQ + s * TILE, &tm_qkv, &sh->q_full[s], w.h * HD, row);
+          tc::bulk_load(sh->lse[s], p.lse2 + stat, BQ * 4, &sh->q_full[s]);
+          tc::bulk_load(sh->delta[s], p.delta + stat, BQ * 4, &sh->q_full[s]);
+        }
+        __syncwarp();
+        if (!wait(&sh->do_empty[s], used, 56)) break;
+        if (tc::elect_one()) {
+          tc::mbar_expect_tx(&sh->do_full[s], TILE);
+          load_tile(sDO + s * TILE, &tm_do, &sh->do_full[s], w.h * HD, row);
+        }
+        __syncwarp();
+        if (i == 0) {
+          // K: every product of the item before has completed; V: its tile staged that item's dV
+          if (j > 0 && !wait(&sh->fin, (uint32_t)j - 1, 59)) break;
+          if (tc::elect_one()) {
+            tc::mbar_expect_tx(&sh->k_full, TILE);
+            load_tile(sK, &tm_qkv, &sh->k_full, H + w.h * HD, w.key0);
+          }
+          __syncwarp();
+          if (j > 0 && !wait(&sh->st_done, (uint32_t)j - 1, 60)) break;
+          if (tc::elect_one()) {
+            tc::mbar_expect_tx(&sh->v_full, TILE);
+            load_tile(sV, &tm_qkv, &sh->v_full, 2 * H + w.h * HD, w.key0);
+          }
+          __syncwarp();
+        }
       }
-      __syncwarp();
-      if (!wait(&sh->do_empty[s], par2, 56)) break;
-      if (tc::elect_one()) {
-        tc::mbar_expect_tx(&sh->do_full[s], TILE);
-        load_tile(sDO + s * TILE, &tm_do, &sh->do_full[s], q_col, row);
-      }
-      __syncwarp();
     }
     // Nothing may land after the CTA has left: the issuer has waited for every full barrier of
     // the loads above unless a wait ran out.
@@ -1513,7 +1563,10 @@ static int launch_bwd(const void* qkv, const void* out, const void* d_out, const
       return 1005;
     CUtensorMap tm_dkv;
     if (make_map(&tm_dkv, dqkv, tokens, 3 * H, 64, 128)) return 1008;
-    attention_bwd_pipelined_kernel<HD><<<grid, kBwdPipeThreads, BwdPipe<HD>::SMEM, st>>>(
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    attention_bwd_pipelined_kernel<HD><<<grid < sms ? grid : sms, kBwdPipeThreads, BwdPipe<HD>::SMEM, st>>>(
         tm_qkv, tm_do, tm_dq, tm_dkv, p);
   } else {
     const int rc = tma_dq ? launch_bwd_kernel<HD, true>(tm_qkv, tm_do, tm_dq, p, grid, st)

@@ -7,6 +7,7 @@
 
 #define __host__
 #define __device__
+#include "attention_schedule.cuh"
 #include "gemm_schedule.cuh"
 
 template <int BM, int BN>
@@ -42,6 +43,16 @@ int main() {
     }
     checked += 2;
   }
+  // persistent attention: every item once, a CTA's items end at the first index past the end
+  for (int ctas = 1; ctas <= 150; ctas += 7)
+    for (int total = ctas; total <= 1100; total += 37) {
+      std::vector<int> taken(total, 0);
+      for (int c = 0; c < ctas; ++c)
+        for (int j = 0; attn_sched::item_index(c, ctas, j) < total; ++j)
+          ++taken[attn_sched::item_index(c, ctas, j)];
+      for (int t : taken)
+        if (t != 1) return 9;
+    }
   // shares of K: in order, without gaps, none empty
   for (int kb = 1; kb <= 200; ++kb)
     for (int splits = 1; splits <= 8 && splits <= kb; ++splits)
