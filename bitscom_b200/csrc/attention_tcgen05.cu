@@ -609,6 +609,329 @@ attention_fwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_q,    // b
 }
 
 // ---------------------------------------------------------------------------
+// forward, two query tiles per CTA
+// ---------------------------------------------------------------------------
+// One persistent CTA per SM works on 256 query rows at a time as two tiles of 128, each with its
+// own softmax warps and its own issuer, so that the matrix products of one tile run under the
+// exponentials of the other (per 128 x 128 block: 1.0 k cycles of products at head_dim 128 and
+// 1.0 k cycles of the special-function unit, which is the floor).  Against the kernel above:
+//   * 128 keys per block instead of 64, P (bf16) goes back into tensor memory over the scores its
+//     thread has read and is the A operand of P V from there: no shared-memory round trip;
+//   * O is rescaled only when a row maximum has grown by more than 2^8: until then the old
+//     reference serves (P and its sum grow by that factor, both are relative to the same
+//     reference, P keeps its eight significant bits);
+//   * K and V tiles are a ring that both tiles read and that runs on into the next item; O leaves
+//     through the tile's Q buffer as whole lines.
+// warps 0-3 softmax of tile 0, 4-7 of tile 1 (thread <-> query row), 8 / 9 issuers, 10 loader.
+// Why each buffer may be written when it is (t: tile, c: running block number of the tile):
+//   S_t (and P_t over it)  QK(c) is issued after o_done[t](c - 1)
+//   O_t                    rescaled between s_full[t](c) and p_full[t](c): PV(c - 1) is complete
+//                          and PV(c) not issued; the next item's PV after o_drained[t]
+//   Q_t                    staging after the last o_done[t]; loaded after q_empty[t]
+//   ring slot              loaded after both issuers have released it
+constexpr int kDualThreads = 11 * 32;
+
+template <int HD> struct FwdDual {
+  static constexpr int TILE = 128 * HD * 2;               // Q, K, V tile: 128 rows x HD
+  static constexpr int STAGES = HD == 128 ? 5 : 8;
+  static constexpr int DATA = (2 + STAGES) * TILE;
+  static constexpr int SMEM = DATA + 512;
+};
+struct DualShared {
+  uint64_t full[8], empty[8];
+  uint64_t q_full[2], q_empty[2], s_full[2], p_full[2], o_done[2], o_drained[2];
+  uint32_t tmem_base;
+  volatile int abort;
+};
+static_assert(sizeof(DualShared) <= 512, "barriers fit behind the tiles");
+
+template <int HD>
+__global__ void __launch_bounds__(kDualThreads, 1)
+attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {64, 128}
+                          const __grid_constant__ CUtensorMap tm_out,  // box {64, 32}
+                          const FwdParams p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  constexpr int TILE = FwdDual<HD>::TILE, STAGES = FwdDual<HD>::STAGES;
+  uint8_t* sQ = smem;
+  uint8_t* sKV = sQ + 2 * TILE;
+  DualShared* sh = reinterpret_cast<DualShared*>(smem + FwdDual<HD>::DATA);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if ((tc::smem_u32(smem) & 1023u) != 0u) {  // same answer in every thread of the CTA
+    if (tid == 0) record_fail(70);
+    return;
+  }
+  const int H = p.heads * HD;
+  const int qblocks = p.seq / BQ, pairs = (qblocks + 1) / 2, bhs = p.batch * p.heads;
+
+  if (tid == 0) {
+    for (int i = 0; i < STAGES; ++i) {
+      tc::mbar_init(&sh->full[i], 1);
+      tc::mbar_init(&sh->empty[i], 2);
+    }
+    for (int t = 0; t < 2; ++t) {
+      tc::mbar_init(&sh->q_full[t], 1);
+      tc::mbar_init(&sh->q_empty[t], 4);
+      tc::mbar_init(&sh->s_full[t], 1);
+      tc::mbar_init(&sh->p_full[t], 4);
+      tc::mbar_init(&sh->o_done[t], 1);
+      tc::mbar_init(&sh->o_drained[t], 4);
+    }
+    sh->abort = 0;
+    tc::fence_mbar_init();
+  }
+  if (warp == 8) tc::tmem_alloc(&sh->tmem_base, 512);
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  tc::tc_fence_after_sync();
+  const uint32_t tmem = sh->tmem_base;
+
+  bool ok = true;
+  auto wait = [&](uint64_t* bar, uint32_t parity, unsigned code) {
+    if (ok && !tc::mbar_wait_warp(bar, parity & 1u, kBudgetNs)) {
+      ok = false;
+      if (lane == 0) {
+        sh->abort = 1;
+        record_fail(code);
+      }
+    }
+    return ok;
+  };
+  auto arrive = [&](uint64_t* bar) {  // once per warp, after every lane's accesses
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(bar);
+  };
+
+  // Item: query rows [256 m, 256 m + 256) of one (batch, head); the tiles have n0 and n1 key
+  // blocks (n1 = 0 where an odd number of query blocks leaves the last pair without its second).
+  struct Item {
+    int m, b, h, n[2], nk;
+  };
+  auto item = [&](int j, Item& w) {
+    const int t = attn_sched::item_index((int)blockIdx.x, (int)gridDim.x, j);
+    if (t >= pairs * bhs) return false;
+    w.m = pairs - 1 - t / bhs;
+    const int bh = t % bhs;
+    w.h = bh % p.heads;
+    w.b = bh / p.heads;
+    w.n[0] = 2 * w.m + 1;
+    w.n[1] = 2 * w.m + 1 < qblocks ? 2 * w.m + 2 : 0;
+    w.nk = w.n[1] ? w.n[1] : w.n[0];
+    return true;
+  };
+  Item w;
+
+  if (warp < 8) {
+    // ------------------------------- softmax ------------------------------------------
+    const int t = warp >> 2;
+    const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tS = tmem + t * 128 + lane_addr, tO = tmem + 256 + t * HD + lane_addr;
+    const int row = ((warp & 3) << 5) | lane;
+    uint32_t c = 0;
+    for (int j = 0; ok && item(j, w); ++j) {
+      const int n = t ? w.n[1] : w.n[0];
+      if (n == 0) continue;
+      float m_run = -INFINITY, l_run = 0.0f;
+      for (int i = 0; i < n; ++i, ++c) {
+        if (!wait(&sh->s_full[t], c, 71)) break;
+        tc::tc_fence_after_sync();
+        float s[128];  // raw scores, then probabilities
+        {
+          uint32_t r[128];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            tc::tmem_ld_32x32(tS + q * 32, reinterpret_cast<uint32_t(&)[32]>(r[q * 32]));
+          tc::tmem_wait_ld();
+#pragma unroll
+          for (int q = 0; q < 128; ++q) s[q] = __uint_as_float(r[q]);
+        }
+        if (i == n - 1) {  // the block on the diagonal
+#pragma unroll
+          for (int q = 0; q < 128; ++q)
+            if (q > row) s[q] = -INFINITY;
+        }
+        // the softmax scale is positive, so the maximum can be taken on the raw scores
+        float mx[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+        for (int q = 4; q < 128; q += 4) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], s[q + u]);
+        }
+        const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
+        if (i == 0) {
+          m_run = m_blk;
+        } else if (__any_sync(0xffffffffu, m_blk > m_run + 8.0f)) {
+          const float m_new = fmaxf(m_run, m_blk);
+          const float alpha = ex2_fast(m_run - m_new);
+          l_run *= alpha;
+          m_run = m_new;
+#pragma unroll 1
+          for (int q = 0; q < HD / 32; ++q) {
+            uint32_t r[32];
+            tc::tmem_ld_32x32(tO + q * 32, r);
+            tc::tmem_wait_ld();
+#pragma unroll
+            for (int u = 0; u < 32; ++u) r[u] = __float_as_uint(__uint_as_float(r[u]) * alpha);
+            tc::tmem_st_32x32(tO + q * 32, r);
+          }
+        }
+        float sm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t pk[32];
+#pragma unroll
+          for (int q = 0; q < 64; q += 4) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              float& x = s[hf * 64 + q + u];
+              x = ex2_fast(fmaf(x, p.scale_log2, -m_run));
+              sm[u] += x;
+            }
+            pk[q / 2] = pack_bf16(s[hf * 64 + q], s[hf * 64 + q + 1]);
+            pk[q / 2 + 1] = pack_bf16(s[hf * 64 + q + 2], s[hf * 64 + q + 3]);
+          }
+          tc::tmem_st_32x32(tS + hf * 32, pk);
+        }
+        l_run += (sm[0] + sm[1]) + (sm[2] + sm[3]);
+        tc::tmem_wait_st();
+        tc::tc_fence_before_sync();
+        arrive(&sh->p_full[t]);
+      }
+      // ---- O / l -> out, through the tile's Q buffer ----
+      if (!wait(&sh->o_done[t], c - 1, 72)) break;
+      tc::tc_fence_after_sync();
+      const float inv = 1.0f / l_run;
+      uint8_t* stage = sQ + t * TILE;
+#pragma unroll
+      for (int q = 0; q < HD / 32; ++q) {
+        uint32_t r[32];
+        tc::tmem_ld_32x32(tO + q * 32, r);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          *reinterpret_cast<uint4*>(stage + (q >> 1) * 128 * 128 + swz(row, (q & 1) * 4 + u)) =
+              make_uint4(
+                  pack_bf16(__uint_as_float(r[u * 8 + 0]) * inv, __uint_as_float(r[u * 8 + 1]) * inv),
+                  pack_bf16(__uint_as_float(r[u * 8 + 2]) * inv, __uint_as_float(r[u * 8 + 3]) * inv),
+                  pack_bf16(__uint_as_float(r[u * 8 + 4]) * inv, __uint_as_float(r[u * 8 + 5]) * inv),
+                  pack_bf16(__uint_as_float(r[u * 8 + 6]) * inv, __uint_as_float(r[u * 8 + 7]) * inv));
+      }
+      tc::tc_fence_before_sync();
+      arrive(&sh->o_drained[t]);
+      const int q_idx = (2 * w.m + t) * BQ + row;
+      p.lse2[((size_t)w.b * p.heads + w.h) * p.seq + q_idx] = m_run + log2f(l_run);
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) {
+        const int out_row = w.b * p.seq + (2 * w.m + t) * BQ + (warp & 3) * 32;
+#pragma unroll
+        for (int q = 0; q < HD / 64; ++q)
+          tc::tma_store_2d(&tm_out, stage + q * 128 * 128 + (warp & 3) * 4096, w.h * HD + 64 * q,
+                           out_row);
+        tc::bulk_commit_group();
+        tc::bulk_wait_group_read0();
+      }
+      arrive(&sh->q_empty[t]);
+    }
+    if (lane == 0) tc::bulk_wait_group0();
+    __syncwarp();
+  } else if (warp < 10) {
+    // ------------------------------- issuers --------------------------------------------
+    const int t = warp - 8;
+    constexpr uint32_t idesc_s = tc::make_idesc_bf16(128, 128, false, false);
+    constexpr uint32_t idesc_o = tc::make_idesc_bf16(128, HD, false, true);
+    constexpr uint32_t hi = tc::desc_hi(1024);
+    constexpr uint32_t CH = 128 * 128;  // bytes between 64-column chunks
+    const uint32_t tS = tmem + t * 128, tO = tmem + 256 + t * HD;
+    const uint32_t q_lo = tc::desc_lo(tc::smem_u32(sQ + t * TILE), 16);
+    const uint32_t kv = tc::smem_u32(sKV);
+    uint32_t c = 0, items = 0, r = 0;  // blocks of this tile, items with this tile, ring fills
+    for (int j = 0; ok && item(j, w); ++j) {
+      const int n = t ? w.n[1] : w.n[0];
+      if (n > 0 && !wait(&sh->q_full[t], items, 73)) break;
+      for (int i = 0; i < w.nk; ++i, r += 2) {
+        const uint32_t ks = r % STAGES, vs = (r + 1) % STAGES;
+        if (!wait(&sh->full[ks], r / STAGES, 74)) break;
+        if (i >= n) {  // only the other tile needs this block
+          arrive(&sh->empty[ks]);
+          if (!wait(&sh->full[vs], (r + 1) / STAGES, 75)) break;
+          arrive(&sh->empty[vs]);
+          continue;
+        }
+        if (c > 0 && !wait(&sh->o_done[t], c - 1, 76)) break;
+        tc::tc_fence_after_sync();
+        const uint32_t k_lo = tc::desc_lo(kv + ks * TILE, 16);
+        if (tc::elect_one()) {
+#pragma unroll
+          for (int s = 0; s < HD / 16; ++s) {
+            const uint32_t step = (uint32_t)((s >> 2) * (CH >> 4) + (s & 3) * 2);
+            tc::umma_bf16_lo<1>(tS, q_lo + step, hi, k_lo + step, hi, idesc_s, s != 0);
+          }
+          tc::umma_commit(&sh->s_full[t]);
+          tc::umma_commit(&sh->empty[ks]);
+        }
+        __syncwarp();
+        if (!wait(&sh->full[vs], (r + 1) / STAGES, 77) || !wait(&sh->p_full[t], c, 78)) break;
+        if (i == 0 && items > 0 && !wait(&sh->o_drained[t], items - 1, 79)) break;
+        tc::tc_fence_after_sync();
+        const uint32_t v_lo = tc::desc_lo(kv + vs * TILE, CH);
+        if (tc::elect_one()) {
+#pragma unroll
+          for (int s = 0; s < 8; ++s)
+            tc::umma_bf16_ta(tO, tS + s * 8, v_lo + s * (16 * 128 >> 4), hi, idesc_o,
+                             (i != 0) || (s != 0));
+          tc::umma_commit(&sh->o_done[t]);
+          tc::umma_commit(&sh->empty[vs]);
+        }
+        __syncwarp();
+        ++c;
+      }
+      items += n > 0;
+    }
+  } else {
+    // ------------------------------- loader ----------------------------------------------
+    auto load_tile = [&](uint8_t* dst, uint64_t* bar, int col, int row) {
+      if (tc::elect_one()) {
+        tc::mbar_expect_tx(bar, TILE);
+#pragma unroll
+        for (int q = 0; q < HD / 64; ++q)
+          tc::tma_load_2d(dst + q * 128 * 128, &tm_qkv, bar, col + 64 * q, row);
+      }
+      __syncwarp();
+    };
+    uint32_t r = 0, items[2] = {0, 0};
+    for (int j = 0; ok && item(j, w); ++j) {
+      const int row0 = w.b * p.seq;
+      for (int i = 0; i < w.nk; ++i) {
+#pragma unroll
+        for (int v = 0; v < 2; ++v, ++r) {  // K, then V of block i
+          const uint32_t slot = r % STAGES;
+          if (!wait(&sh->empty[slot], r / STAGES + 1, 80)) break;
+          load_tile(sKV + slot * TILE, &sh->full[slot], (1 + v) * H + w.h * HD, row0 + i * 128);
+        }
+        if (!ok) break;
+        if (i == 0) {  // behind the first K and V, which need not wait for the item before
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (w.n[t] == 0) continue;
+            if (!wait(&sh->q_empty[t], items[t] + 1, 81)) break;
+            load_tile(sQ + t * TILE, &sh->q_full[t], w.h * HD, row0 + (2 * w.m + t) * BQ);
+            ++items[t];
+          }
+        }
+      }
+    }
+    // every load has been waited for by an issuer before the CTA leaves, unless a wait ran out
+  }
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 8) {
+    tc::tc_fence_after_sync();
+    tc::tmem_dealloc(tmem, 512);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // backward
 // ---------------------------------------------------------------------------
 struct BwdParams {
@@ -1466,8 +1789,33 @@ static int launch_fwd(const void* qkv, void* out, void* lse2, int batch, int seq
 // 0: float4 atomics, 1: TMA reduce-add from shared memory, 2: the software-pipelined kernel (which
 // reduces by TMA as well)
 static int g_bwd_dq_variant = 2;
-// 0: attention_fwd_kernel, 1: attention_fwd_pipelined_kernel
-static int g_fwd_variant = 1;
+// 0: attention_fwd_kernel, 1: attention_fwd_pipelined_kernel, 2: attention_fwd_dual_kernel
+static int g_fwd_variant = 2;
+
+template <int HD>
+static int launch_fwd_dual(const void* qkv, void* out, void* lse2, int batch, int seq, int heads,
+                           float scale, cudaStream_t st) {
+  const long long tokens = (long long)batch * seq;
+  CUtensorMap tm_qkv, tm_out;
+  if (make_map(&tm_qkv, qkv, tokens, 3 * heads * HD, 64, 128)) return 1003;
+  if (make_map(&tm_out, out, tokens, heads * HD, 64, 32)) return 1008;
+  if (!tc::ensure_dynamic_smem((const void*)attention_fwd_dual_kernel<HD>, FwdDual<HD>::SMEM))
+    return 1005;
+  FwdParams p;
+  p.out = (__nv_bfloat16*)out;
+  p.lse2 = (float*)lse2;
+  p.batch = batch;
+  p.seq = seq;
+  p.heads = heads;
+  p.scale_log2 = scale * kLog2e;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int items = batch * heads * ((seq / BQ + 1) / 2);
+  attention_fwd_dual_kernel<HD><<<items < sms ? items : sms, kDualThreads, FwdDual<HD>::SMEM, st>>>(
+      tm_qkv, tm_out, p);
+  return (int)cudaGetLastError();
+}
 
 template <int HD>
 static int launch_fwd_pipelined(const void* qkv, void* out, void* lse2, int batch, int seq,
@@ -1611,6 +1959,9 @@ int bcom_attention_fwd(const void* qkv, void* out, void* lse2, int batch, int se
   if (((uintptr_t)qkv & 15) || ((uintptr_t)out & 15)) return 1002;
   tc::bind_context_once();
   cudaStream_t st = (cudaStream_t)stream;
+  if (g_fwd_variant == 2)
+    return head_dim == 128 ? launch_fwd_dual<128>(qkv, out, lse2, batch, seq, heads, scale, st)
+                           : launch_fwd_dual<64>(qkv, out, lse2, batch, seq, heads, scale, st);
   if (g_fwd_variant == 1)
     return head_dim == 128
                ? launch_fwd_pipelined<128>(qkv, out, lse2, batch, seq, heads, scale, st)
@@ -1620,10 +1971,11 @@ int bcom_attention_fwd(const void* qkv, void* out, void* lse2, int batch, int se
 }
 
 // 0 selects the forward kernel whose MMA and softmax take turns, 1 the software-pipelined one
-// (issuer warp, double-buffered S in TMEM, O accumulated in TMEM).  Returns the previous value.
+// (issuer warp, double-buffered S in TMEM, O accumulated in TMEM), 2 the one with two query tiles
+// per persistent CTA (default).  Returns the previous value.
 int bcom_attention_set_fwd_variant(int variant) {
   const int old = attn::g_fwd_variant;
-  if (variant >= 0 && variant <= 1) attn::g_fwd_variant = variant;
+  if (variant >= 0 && variant <= 2) attn::g_fwd_variant = variant;
   return old;
 }
 

@@ -17,8 +17,9 @@ from ._native import NativeError, check, ptr, stream_ptr
 _lib = None
 _scratch: Dict[Tuple, torch.Tensor] = {}
 # forward kernels: "simple" alternates MMA and softmax inside a CTA; "pipelined" has an issuer
-# warp, double-buffered scores in TMEM and the output accumulated in TMEM
-_FWD_VARIANTS = {"simple": 0, "pipelined": 1}
+# warp, double-buffered scores in TMEM and the output accumulated in TMEM; "dual" (default) has
+# two query tiles per persistent CTA whose products and softmax overlap
+_FWD_VARIANTS = {"simple": 0, "pipelined": 1, "dual": 2}
 # backward kernels: MMA groups and softmax take turns and a dQ tile is added to the fp32
 # accumulator by float4 atomics from registers or by TMA reductions from a staging tile, or the
 # software-pipelined kernel (default; TMA reductions as well)
@@ -53,15 +54,15 @@ def available() -> bool:
 
 
 def set_forward_variant(name: str) -> str:
-    """Select the forward kernel ("simple" or "pipelined", also ``BITSCOM_ATTN_FWD``); returns
-    the name that was active before."""
+    """Select the forward kernel ("simple", "pipelined" or "dual", also
+    ``BITSCOM_ATTN_FWD``); returns the name that was active before."""
     if name not in _FWD_VARIANTS:
         raise ValueError(f"unknown attention forward variant {name!r}")
     lib = _get()
     if lib is None:
         raise NativeError("attention kernel needs the bcom_llama library and a GPU")
     old = lib.bcom_attention_set_fwd_variant(_FWD_VARIANTS[name])
-    return {0: "simple", 1: "pipelined"}[old]
+    return {0: "simple", 1: "pipelined", 2: "dual"}[old]
 
 
 def set_backward_dq_variant(name: str) -> str:
