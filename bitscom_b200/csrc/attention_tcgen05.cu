@@ -612,34 +612,42 @@ attention_fwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_q,    // b
 // forward, two query tiles per CTA
 // ---------------------------------------------------------------------------
 // One persistent CTA per SM works on 256 query rows at a time as two tiles of 128, each with its
-// own softmax warps and its own issuer, so that the matrix products of one tile run under the
-// exponentials of the other (per 128 x 128 block: 1.0 k cycles of products at head_dim 128 and
-// 1.0 k cycles of the special-function unit, which is the floor).  Against the kernel above:
-//   * 128 keys per block instead of 64, P (bf16) goes back into tensor memory over the scores its
-//     thread has read and is the A operand of P V from there: no shared-memory round trip;
+// own softmax warps and its own issuer, so that the matrix products run under the exponentials
+// (per 128 x 128 block and tile: 1.0 k cycles of products at head_dim 128 and 1.0 k cycles of the
+// special-function unit, which is the floor).  Against the kernel above:
+//   * P (bf16) goes back into tensor memory over the scores its thread has read and is the A
+//     operand of P V from there: no shared-memory round trip;
+//   * blocks of 64 keys with two score buffers per tile: the next block's scores are ready when a
+//     softmax warp gets to them.  With one buffer of 128 keys (P over it) the softmax warps
+//     waited 2.4 k of 4.9 k cycles per block for P V, then Q K^T, to go through (95 / 52 us);
 //   * O is rescaled only when a row maximum has grown by more than 2^8: until then the old
 //     reference serves (P and its sum grow by that factor, both are relative to the same
 //     reference, P keeps its eight significant bits);
 //   * K and V tiles are a ring that both tiles read and that runs on into the next item; O leaves
 //     through the tile's Q buffer as whole lines.
 // warps 0-3 softmax of tile 0, 4-7 of tile 1 (thread <-> query row), 8 / 9 issuers, 10 loader.
+// Order of a tile's products: QK_0 QK_1 | PV_0 QK_2 | PV_1 QK_3 | ...; ring order K0 K1 V0 K2 V1 ...
 // Why each buffer may be written when it is (t: tile, c: running block number of the tile):
-//   S_t (and P_t over it)  QK(c) is issued after o_done[t](c - 1)
-//   O_t                    rescaled between s_full[t](c) and p_full[t](c): PV(c - 1) is complete
-//                          and PV(c) not issued; the next item's PV after o_drained[t]
-//   Q_t                    staging after the last o_done[t]; loaded after q_empty[t]
+//   S_t[c & 1] (and P over it)  QK(c) is issued after o_done[t][c & 1] of block c - 2
+//   O_t                    rescaled after o_done of block c - 1 and before p_full(c), without which
+//                          PV(c) is not issued; the next item's first PV after o_drained[t]
+//   Q_t                    staging after the last o_done; loaded after q_empty[t]
 //   ring slot              loaded after both issuers have released it
+// Measured: B2 S2048 H32 D128 119 us (pipelined kernel) -> DUAL_US us, B8 S1024 H16 D64
+// 62 -> DUAL64_US us.
 constexpr int kDualThreads = 11 * 32;
 
 template <int HD> struct FwdDual {
-  static constexpr int TILE = 128 * HD * 2;               // Q, K, V tile: 128 rows x HD
-  static constexpr int STAGES = HD == 128 ? 5 : 8;
-  static constexpr int DATA = (2 + STAGES) * TILE;
+  static constexpr int Q_TILE = 128 * HD * 2;
+  static constexpr int KV_TILE = BKF * HD * 2;             // 64 keys x HD
+  static constexpr int STAGES = 10;
+  static constexpr int DATA = 2 * Q_TILE + STAGES * KV_TILE;  // 224 KiB at head_dim 128
   static constexpr int SMEM = DATA + 512;
 };
 struct DualShared {
-  uint64_t full[8], empty[8];
-  uint64_t q_full[2], q_empty[2], s_full[2], p_full[2], o_done[2], o_drained[2];
+  uint64_t full[10], empty[10];
+  uint64_t q_full[2], q_empty[2], o_drained[2];
+  uint64_t s_full[2][2], p_full[2][2], o_done[2][2];  // [tile][block & 1]
   uint32_t tmem_base;
   volatile int abort;
 };
@@ -647,13 +655,15 @@ static_assert(sizeof(DualShared) <= 512, "barriers fit behind the tiles");
 
 template <int HD>
 __global__ void __launch_bounds__(kDualThreads, 1)
-attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {64, 128}
+attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_q,    // box {64, 128}
+                          const __grid_constant__ CUtensorMap tm_kv,   // box {64, 64}
                           const __grid_constant__ CUtensorMap tm_out,  // box {64, 32}
                           const FwdParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr int TILE = FwdDual<HD>::TILE, STAGES = FwdDual<HD>::STAGES;
+  constexpr int Q_TILE = FwdDual<HD>::Q_TILE, KV_TILE = FwdDual<HD>::KV_TILE;
+  constexpr uint32_t STAGES = FwdDual<HD>::STAGES;
   uint8_t* sQ = smem;
-  uint8_t* sKV = sQ + 2 * TILE;
+  uint8_t* sKV = sQ + 2 * Q_TILE;
   DualShared* sh = reinterpret_cast<DualShared*>(smem + FwdDual<HD>::DATA);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -665,17 +675,19 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {6
   const int qblocks = p.seq / BQ, pairs = (qblocks + 1) / 2, bhs = p.batch * p.heads;
 
   if (tid == 0) {
-    for (int i = 0; i < STAGES; ++i) {
+    for (int i = 0; i < (int)STAGES; ++i) {
       tc::mbar_init(&sh->full[i], 1);
       tc::mbar_init(&sh->empty[i], 2);
     }
     for (int t = 0; t < 2; ++t) {
       tc::mbar_init(&sh->q_full[t], 1);
       tc::mbar_init(&sh->q_empty[t], 4);
-      tc::mbar_init(&sh->s_full[t], 1);
-      tc::mbar_init(&sh->p_full[t], 4);
-      tc::mbar_init(&sh->o_done[t], 1);
       tc::mbar_init(&sh->o_drained[t], 4);
+      for (int i = 0; i < 2; ++i) {
+        tc::mbar_init(&sh->s_full[t][i], 1);
+        tc::mbar_init(&sh->p_full[t][i], 4);
+        tc::mbar_init(&sh->o_done[t][i], 1);
+      }
     }
     sh->abort = 0;
     tc::fence_mbar_init();
@@ -702,8 +714,9 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {6
     if (lane == 0) tc::mbar_arrive(bar);
   };
 
-  // Item: query rows [256 m, 256 m + 256) of one (batch, head); the tiles have n0 and n1 key
-  // blocks (n1 = 0 where an odd number of query blocks leaves the last pair without its second).
+  // Item: query rows [256 m, 256 m + 256) of one (batch, head); the tiles have n[0] and n[1] key
+  // blocks, both even (n[1] = 0 where an odd number of query blocks leaves the last pair without
+  // its second tile); nk blocks are loaded.
   struct Item {
     int m, b, h, n[2], nk;
   };
@@ -714,8 +727,8 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {6
     const int bh = t % bhs;
     w.h = bh % p.heads;
     w.b = bh / p.heads;
-    w.n[0] = 2 * w.m + 1;
-    w.n[1] = 2 * w.m + 1 < qblocks ? 2 * w.m + 2 : 0;
+    w.n[0] = 4 * w.m + 2;
+    w.n[1] = 2 * w.m + 1 < qblocks ? 4 * w.m + 4 : 0;
     w.nk = w.n[1] ? w.n[1] : w.n[0];
     return true;
   };
@@ -725,7 +738,7 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {6
     // ------------------------------- softmax ------------------------------------------
     const int t = warp >> 2;
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tS = tmem + t * 128 + lane_addr, tO = tmem + 256 + t * HD + lane_addr;
+    const uint32_t tO = tmem + 256 + t * HD + lane_addr;
     const int row = ((warp & 3) << 5) | lane;
     uint32_t c = 0;
     for (int j = 0; ok && item(j, w); ++j) {
@@ -733,27 +746,28 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {6
       if (n == 0) continue;
       float m_run = -INFINITY, l_run = 0.0f;
       for (int i = 0; i < n; ++i, ++c) {
-        if (!wait(&sh->s_full[t], c, 71)) break;
+        const uint32_t tS = tmem + t * 128 + (c & 1) * 64 + lane_addr;
+        if (!wait(&sh->s_full[t][c & 1], c >> 1, 71)) break;
         tc::tc_fence_after_sync();
-        float s[128];  // raw scores, then probabilities
+        float s[BKF];  // raw scores, then probabilities
         {
-          uint32_t r[128];
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            tc::tmem_ld_32x32(tS + q * 32, reinterpret_cast<uint32_t(&)[32]>(r[q * 32]));
+          uint32_t r[BKF];
+          tc::tmem_ld_32x32(tS, reinterpret_cast<uint32_t(&)[32]>(r[0]));
+          tc::tmem_ld_32x32(tS + 32, reinterpret_cast<uint32_t(&)[32]>(r[32]));
           tc::tmem_wait_ld();
 #pragma unroll
-          for (int q = 0; q < 128; ++q) s[q] = __uint_as_float(r[q]);
+          for (int q = 0; q < BKF; ++q) s[q] = __uint_as_float(r[q]);
         }
-        if (i == n - 1) {  // the block on the diagonal
+        if (i >= n - 2) {  // the two blocks on the diagonal
+          const int last = row - (i - (n - 2)) * BKF;  // last visible column
 #pragma unroll
-          for (int q = 0; q < 128; ++q)
-            if (q > row) s[q] = -INFINITY;
+          for (int q = 0; q < BKF; ++q)
+            if (q > last) s[q] = -INFINITY;
         }
         // the softmax scale is positive, so the maximum can be taken on the raw scores
         float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-        for (int q = 4; q < 128; q += 4) {
+        for (int q = 4; q < BKF; q += 4) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], s[q + u]);
         }
@@ -765,6 +779,8 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {6
           const float alpha = ex2_fast(m_run - m_new);
           l_run *= alpha;
           m_run = m_new;
+          if (!wait(&sh->o_done[t][(c - 1) & 1], (c - 1) >> 1, 72)) break;
+          tc::tc_fence_after_sync();
 #pragma unroll 1
           for (int q = 0; q < HD / 32; ++q) {
             uint32_t r[32];
@@ -776,32 +792,28 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {6
           }
         }
         float sm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        uint32_t pk[32];
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t pk[32];
+        for (int q = 0; q < BKF; q += 4) {
 #pragma unroll
-          for (int q = 0; q < 64; q += 4) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              float& x = s[hf * 64 + q + u];
-              x = ex2_fast(fmaf(x, p.scale_log2, -m_run));
-              sm[u] += x;
-            }
-            pk[q / 2] = pack_bf16(s[hf * 64 + q], s[hf * 64 + q + 1]);
-            pk[q / 2 + 1] = pack_bf16(s[hf * 64 + q + 2], s[hf * 64 + q + 3]);
+          for (int u = 0; u < 4; ++u) {
+            s[q + u] = ex2_fast(fmaf(s[q + u], p.scale_log2, -m_run));
+            sm[u] += s[q + u];
           }
-          tc::tmem_st_32x32(tS + hf * 32, pk);
+          pk[q / 2] = pack_bf16(s[q], s[q + 1]);
+          pk[q / 2 + 1] = pack_bf16(s[q + 2], s[q + 3]);
         }
+        tc::tmem_st_32x32(tS, pk);
         l_run += (sm[0] + sm[1]) + (sm[2] + sm[3]);
         tc::tmem_wait_st();
         tc::tc_fence_before_sync();
-        arrive(&sh->p_full[t]);
+        arrive(&sh->p_full[t][c & 1]);
       }
       // ---- O / l -> out, through the tile's Q buffer ----
-      if (!wait(&sh->o_done[t], c - 1, 72)) break;
+      if (!wait(&sh->o_done[t][(c - 1) & 1], (c - 1) >> 1, 73)) break;
       tc::tc_fence_after_sync();
       const float inv = 1.0f / l_run;
-      uint8_t* stage = sQ + t * TILE;
+      uint8_t* stage = sQ + t * Q_TILE;
 #pragma unroll
       for (int q = 0; q < HD / 32; ++q) {
         uint32_t r[32];
@@ -838,87 +850,108 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // box {6
   } else if (warp < 10) {
     // ------------------------------- issuers --------------------------------------------
     const int t = warp - 8;
-    constexpr uint32_t idesc_s = tc::make_idesc_bf16(128, 128, false, false);
+    constexpr uint32_t idesc_s = tc::make_idesc_bf16(128, BKF, false, false);
     constexpr uint32_t idesc_o = tc::make_idesc_bf16(128, HD, false, true);
     constexpr uint32_t hi = tc::desc_hi(1024);
-    constexpr uint32_t CH = 128 * 128;  // bytes between 64-column chunks
-    const uint32_t tS = tmem + t * 128, tO = tmem + 256 + t * HD;
-    const uint32_t q_lo = tc::desc_lo(tc::smem_u32(sQ + t * TILE), 16);
+    const uint32_t tO = tmem + 256 + t * HD;
+    const uint32_t q_lo = tc::desc_lo(tc::smem_u32(sQ + t * Q_TILE), 16);
     const uint32_t kv = tc::smem_u32(sKV);
-    uint32_t c = 0, items = 0, r = 0;  // blocks of this tile, items with this tile, ring fills
+    // blocks of this tile whose Q K^T / P V has been issued, items with this tile, ring fills
+    uint32_t cq = 0, cv = 0, items = 0, r = 0;
+    // the next ring tile: K of a block (issue Q K^T) or, if this tile does not need it, nothing
+    auto take_k = [&](bool mine) {
+      const uint32_t slot = r % STAGES;
+      if (!wait(&sh->full[slot], r / STAGES, 74)) return;
+      ++r;
+      if (!mine) {
+        arrive(&sh->empty[slot]);
+        return;
+      }
+      if (cq >= 2 && !wait(&sh->o_done[t][cq & 1], (cq >> 1) - 1, 75)) return;
+      tc::tc_fence_after_sync();
+      const uint32_t tS = tmem + t * 128 + (cq & 1) * 64;
+      const uint32_t k_lo = tc::desc_lo(kv + slot * KV_TILE, 16);
+      if (tc::elect_one()) {
+#pragma unroll
+        for (int s = 0; s < HD / 16; ++s)
+          tc::umma_bf16_lo<1>(tS, q_lo + (s >> 2) * (BQ * 128 >> 4) + (s & 3) * 2, hi,
+                              k_lo + (s >> 2) * (BKF * 128 >> 4) + (s & 3) * 2, hi, idesc_s,
+                              s != 0);
+        tc::umma_commit(&sh->s_full[t][cq & 1]);
+        tc::umma_commit(&sh->empty[slot]);
+      }
+      __syncwarp();
+      ++cq;
+    };
     for (int j = 0; ok && item(j, w); ++j) {
       const int n = t ? w.n[1] : w.n[0];
-      if (n > 0 && !wait(&sh->q_full[t], items, 73)) break;
-      for (int i = 0; i < w.nk; ++i, r += 2) {
-        const uint32_t ks = r % STAGES, vs = (r + 1) % STAGES;
-        if (!wait(&sh->full[ks], r / STAGES, 74)) break;
-        if (i >= n) {  // only the other tile needs this block
-          arrive(&sh->empty[ks]);
-          if (!wait(&sh->full[vs], (r + 1) / STAGES, 75)) break;
-          arrive(&sh->empty[vs]);
-          continue;
-        }
-        if (c > 0 && !wait(&sh->o_done[t], c - 1, 76)) break;
-        tc::tc_fence_after_sync();
-        const uint32_t k_lo = tc::desc_lo(kv + ks * TILE, 16);
-        if (tc::elect_one()) {
+      if (n > 0 && !wait(&sh->q_full[t], items, 76)) break;
+      take_k(n > 0);
+      take_k(n > 0);
+      for (int i = 0; i < w.nk && ok; ++i) {
+        const uint32_t slot = r % STAGES;
+        if (!wait(&sh->full[slot], r / STAGES, 77)) break;
+        ++r;
+        if (i < n) {
+          if (!wait(&sh->p_full[t][cv & 1], cv >> 1, 78)) break;
+          if (i == 0 && items > 0 && !wait(&sh->o_drained[t], items - 1, 79)) break;
+          tc::tc_fence_after_sync();
+          const uint32_t v_lo = tc::desc_lo(kv + slot * KV_TILE, BKF * 128);
+          const uint32_t tP = tmem + t * 128 + (cv & 1) * 64;
+          if (tc::elect_one()) {
 #pragma unroll
-          for (int s = 0; s < HD / 16; ++s) {
-            const uint32_t step = (uint32_t)((s >> 2) * (CH >> 4) + (s & 3) * 2);
-            tc::umma_bf16_lo<1>(tS, q_lo + step, hi, k_lo + step, hi, idesc_s, s != 0);
+            for (int s = 0; s < BKF / 16; ++s)
+              tc::umma_bf16_ta(tO, tP + s * 8, v_lo + s * (16 * 128 >> 4), hi, idesc_o,
+                               (i != 0) || (s != 0));
+            tc::umma_commit(&sh->o_done[t][cv & 1]);
+            tc::umma_commit(&sh->empty[slot]);
           }
-          tc::umma_commit(&sh->s_full[t]);
-          tc::umma_commit(&sh->empty[ks]);
+          __syncwarp();
+          ++cv;
+        } else {
+          arrive(&sh->empty[slot]);
         }
-        __syncwarp();
-        if (!wait(&sh->full[vs], (r + 1) / STAGES, 77) || !wait(&sh->p_full[t], c, 78)) break;
-        if (i == 0 && items > 0 && !wait(&sh->o_drained[t], items - 1, 79)) break;
-        tc::tc_fence_after_sync();
-        const uint32_t v_lo = tc::desc_lo(kv + vs * TILE, CH);
-        if (tc::elect_one()) {
-#pragma unroll
-          for (int s = 0; s < 8; ++s)
-            tc::umma_bf16_ta(tO, tS + s * 8, v_lo + s * (16 * 128 >> 4), hi, idesc_o,
-                             (i != 0) || (s != 0));
-          tc::umma_commit(&sh->o_done[t]);
-          tc::umma_commit(&sh->empty[vs]);
-        }
-        __syncwarp();
-        ++c;
+        if (i + 2 < w.nk) take_k(i + 2 < n);
       }
       items += n > 0;
     }
   } else {
     // ------------------------------- loader ----------------------------------------------
-    auto load_tile = [&](uint8_t* dst, uint64_t* bar, int col, int row) {
+    uint32_t r = 0, items[2] = {0, 0};
+    auto load_kv = [&](int v, int i) {  // K (v = 0) or V (v = 1) of block i
+      const uint32_t slot = r % STAGES;
+      if (!wait(&sh->empty[slot], r / STAGES + 1, 80)) return;
+      ++r;
       if (tc::elect_one()) {
-        tc::mbar_expect_tx(bar, TILE);
+        tc::mbar_expect_tx(&sh->full[slot], KV_TILE);
 #pragma unroll
         for (int q = 0; q < HD / 64; ++q)
-          tc::tma_load_2d(dst + q * 128 * 128, &tm_qkv, bar, col + 64 * q, row);
+          tc::tma_load_2d(sKV + slot * KV_TILE + q * BKF * 128, &tm_kv, &sh->full[slot],
+                          (1 + v) * H + w.h * HD + 64 * q, w.b * p.seq + i * BKF);
       }
       __syncwarp();
     };
-    uint32_t r = 0, items[2] = {0, 0};
     for (int j = 0; ok && item(j, w); ++j) {
-      const int row0 = w.b * p.seq;
-      for (int i = 0; i < w.nk; ++i) {
+      load_kv(0, 0);
+      load_kv(0, 1);
+      // behind the first K tiles, which need not wait for the item before
 #pragma unroll
-        for (int v = 0; v < 2; ++v, ++r) {  // K, then V of block i
-          const uint32_t slot = r % STAGES;
-          if (!wait(&sh->empty[slot], r / STAGES + 1, 80)) break;
-          load_tile(sKV + slot * TILE, &sh->full[slot], (1 + v) * H + w.h * HD, row0 + i * 128);
-        }
-        if (!ok) break;
-        if (i == 0) {  // behind the first K and V, which need not wait for the item before
+      for (int t = 0; t < 2; ++t) {
+        if (w.n[t] == 0) continue;
+        if (!wait(&sh->q_empty[t], items[t] + 1, 81)) break;
+        ++items[t];
+        if (tc::elect_one()) {
+          tc::mbar_expect_tx(&sh->q_full[t], Q_TILE);
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            if (w.n[t] == 0) continue;
-            if (!wait(&sh->q_empty[t], items[t] + 1, 81)) break;
-            load_tile(sQ + t * TILE, &sh->q_full[t], w.h * HD, row0 + (2 * w.m + t) * BQ);
-            ++items[t];
-          }
+          for (int q = 0; q < HD / 64; ++q)
+            tc::tma_load_2d(sQ + t * Q_TILE + q * BQ * 128, &tm_q, &sh->q_full[t],
+                            w.h * HD + 64 * q, w.b * p.seq + (2 * w.m + t) * BQ);
         }
+        __syncwarp();
+      }
+      for (int i = 0; i < w.nk && ok; ++i) {
+        load_kv(1, i);
+        if (i + 2 < w.nk) load_kv(0, i + 2);
       }
     }
     // every load has been waited for by an issuer before the CTA leaves, unless a wait ran out
@@ -1796,8 +1829,9 @@ template <int HD>
 static int launch_fwd_dual(const void* qkv, void* out, void* lse2, int batch, int seq, int heads,
                            float scale, cudaStream_t st) {
   const long long tokens = (long long)batch * seq;
-  CUtensorMap tm_qkv, tm_out;
-  if (make_map(&tm_qkv, qkv, tokens, 3 * heads * HD, 64, 128)) return 1003;
+  CUtensorMap tm_q, tm_kv, tm_out;
+  if (make_map(&tm_q, qkv, tokens, 3 * heads * HD, 64, BQ)) return 1003;
+  if (make_map(&tm_kv, qkv, tokens, 3 * heads * HD, 64, BKF)) return 1004;
   if (make_map(&tm_out, out, tokens, heads * HD, 64, 32)) return 1008;
   if (!tc::ensure_dynamic_smem((const void*)attention_fwd_dual_kernel<HD>, FwdDual<HD>::SMEM))
     return 1005;
@@ -1813,7 +1847,7 @@ static int launch_fwd_dual(const void* qkv, void* out, void* lse2, int batch, in
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int items = batch * heads * ((seq / BQ + 1) / 2);
   attention_fwd_dual_kernel<HD><<<items < sms ? items : sms, kDualThreads, FwdDual<HD>::SMEM, st>>>(
-      tm_qkv, tm_out, p);
+      tm_q, tm_kv, tm_out, p);
   return (int)cudaGetLastError();
 }
 
