@@ -620,9 +620,10 @@ attention_fwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_q,    // b
 //   * blocks of 64 keys with two score buffers per tile: the next block's scores are ready when a
 //     softmax warp gets to them.  With one buffer of 128 keys (P over it) the softmax warps
 //     waited 2.4 k of 4.9 k cycles per block for P V, then Q K^T, to go through (95 / 52 us);
-//   * O is rescaled only when a row maximum has grown by more than 2^8: until then the old
-//     reference serves (P and its sum grow by that factor, both are relative to the same
-//     reference, P keeps its eight significant bits);
+//   * O is rescaled after the exponentials, when P V of the block before is through; before them
+//     the softmax warps waited for it (93 / 51 us), in warps of its own the rescaling became the
+//     critical chain (97 / 50 us).  Rescaling only after a maximum has grown by 2^8 takes 80 /
+//     45 us but loses the exact P = 1 of the largest score: 3 % more distance to 64 bits;
 //   * K and V tiles are a ring that both tiles read and that runs on into the next item; O leaves
 //     through the tile's Q buffer as whole lines.
 // warps 0-3 softmax of tile 0, 4-7 of tile 1 (thread <-> query row), 8 / 9 issuers, 10 loader.
@@ -772,25 +773,9 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_q,    // box {6
           for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], s[q + u]);
         }
         const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
-        if (i == 0) {
-          m_run = m_blk;
-        } else if (__any_sync(0xffffffffu, m_blk > m_run + 8.0f)) {
-          const float m_new = fmaxf(m_run, m_blk);
-          const float alpha = ex2_fast(m_run - m_new);
-          l_run *= alpha;
-          m_run = m_new;
-          if (!wait(&sh->o_done[t][(c - 1) & 1], (c - 1) >> 1, 72)) break;
-          tc::tc_fence_after_sync();
-#pragma unroll 1
-          for (int q = 0; q < HD / 32; ++q) {
-            uint32_t r[32];
-            tc::tmem_ld_32x32(tO + q * 32, r);
-            tc::tmem_wait_ld();
-#pragma unroll
-            for (int u = 0; u < 32; ++u) r[u] = __float_as_uint(__uint_as_float(r[u]) * alpha);
-            tc::tmem_st_32x32(tO + q * 32, r);
-          }
-        }
+        const float m_new = fmaxf(m_run, m_blk);
+        const float alpha = ex2_fast(m_run - m_new);  // first block: 2^(-inf) = 0
+        m_run = m_new;
         float sm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         uint32_t pk[32];
 #pragma unroll
@@ -804,7 +789,22 @@ attention_fwd_dual_kernel(const __grid_constant__ CUtensorMap tm_q,    // box {6
           pk[q / 2 + 1] = pack_bf16(s[q + 2], s[q + 3]);
         }
         tc::tmem_st_32x32(tS, pk);
-        l_run += (sm[0] + sm[1]) + (sm[2] + sm[3]);
+        l_run = l_run * alpha + ((sm[0] + sm[1]) + (sm[2] + sm[3]));
+        if (i > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+          if (!wait(&sh->o_done[t][(c - 1) & 1], (c - 1) >> 1, 72)) break;
+          tc::tc_fence_after_sync();
+#pragma unroll
+          for (int q = 0; q < HD / 64; ++q) {
+            uint32_t r[64];
+            tc::tmem_ld_32x32(tO + q * 64, reinterpret_cast<uint32_t(&)[32]>(r[0]));
+            tc::tmem_ld_32x32(tO + q * 64 + 32, reinterpret_cast<uint32_t(&)[32]>(r[32]));
+            tc::tmem_wait_ld();
+#pragma unroll
+            for (int u = 0; u < 64; ++u) r[u] = __float_as_uint(__uint_as_float(r[u]) * alpha);
+            tc::tmem_st_32x32(tO + q * 64, reinterpret_cast<uint32_t(&)[32]>(r[0]));
+            tc::tmem_st_32x32(tO + q * 64 + 32, reinterpret_cast<uint32_t(&)[32]>(r[32]));
+          }
+        }
         tc::tmem_wait_st();
         tc::tc_fence_before_sync();
         arrive(&sh->p_full[t][c & 1]);
@@ -1993,10 +1993,13 @@ int bcom_attention_fwd(const void* qkv, void* out, void* lse2, int batch, int se
   if (((uintptr_t)qkv & 15) || ((uintptr_t)out & 15)) return 1002;
   tc::bind_context_once();
   cudaStream_t st = (cudaStream_t)stream;
-  if (g_fwd_variant == 2)
+  // Two tiles per CTA once there are more tiles than SMs: below that a CTA per tile uses more of
+  // the chip (B1 S2048 H8 D128, 128 tiles: 36.5 us against 41.3; B4 S512 H16 D64, 256 tiles: 14.4
+  // against 12.5; B2 S1024 H32 D128, 512 tiles: 46 against 33).
+  if (g_fwd_variant == 2 && (long long)batch * heads * (seq / BQ) > 148)
     return head_dim == 128 ? launch_fwd_dual<128>(qkv, out, lse2, batch, seq, heads, scale, st)
                            : launch_fwd_dual<64>(qkv, out, lse2, batch, seq, heads, scale, st);
-  if (g_fwd_variant == 1)
+  if (g_fwd_variant >= 1)
     return head_dim == 128
                ? launch_fwd_pipelined<128>(qkv, out, lse2, batch, seq, heads, scale, st)
                : launch_fwd_pipelined<64>(qkv, out, lse2, batch, seq, heads, scale, st);
@@ -2006,7 +2009,7 @@ int bcom_attention_fwd(const void* qkv, void* out, void* lse2, int batch, int se
 
 // 0 selects the forward kernel whose MMA and softmax take turns, 1 the software-pipelined one
 // (issuer warp, double-buffered S in TMEM, O accumulated in TMEM), 2 the one with two query tiles
-// per persistent CTA (default).  Returns the previous value.
+// per persistent CTA (default; few tiles take 1).  Returns the previous value.
 int bcom_attention_set_fwd_variant(int variant) {
   const int old = attn::g_fwd_variant;
   if (variant >= 0 && variant <= 2) attn::g_fwd_variant = variant;

@@ -104,6 +104,35 @@ def test_backward_dq_variants_match_reference(B, S, nh, hd, dq):
         A.set_backward_dq_variant(before)
 
 
+@pytest.mark.parametrize("hd", [128, 64])
+@pytest.mark.parametrize("B,S,nh,growth", [(19, 128, 8, 0.0), (10, 384, 6, 0.0), (2, 1024, 10, 4.0)])
+def test_persistent_kernels_match_reference(B, S, nh, growth, hd):
+    """More tiles than SMs: the two-tile forward kernel and the persistent backward kernel, whose
+    CTAs take several items each; single-block items, an odd number of query blocks (last pair
+    without its second tile), and keys that grow along the sequence, so that the row maxima rise
+    in every block.  bf16 P and output: 2^-8 relative of the largest value, with a factor 4."""
+    H = nh * hd
+    g = torch.Generator(device="cuda").manual_seed(B + S + hd)
+    qkv = torch.randn(B * S, 3 * H, device="cuda", generator=g) * 0.7
+    qkv[:, H:2 * H] *= (1 + growth * torch.arange(S, device="cuda") / S).repeat(B)[:, None]
+    qkv = qkv.to(torch.bfloat16)
+    d_out = (torch.randn(B * S, H, device="cuda", generator=g) * 0.5).to(torch.bfloat16)
+    assert B * nh * (S // 128) > 148
+    x = qkv.clone().requires_grad_()
+    out = A.attention(x, B, S, nh, hd)
+    out.backward(d_out)
+    torch.cuda.synchronize()
+    A.check_status()
+    xr = qkv.float().requires_grad_()
+    ref = _ref(xr, B, S, nh, hd)
+    ref.backward(d_out.float())
+    assert (out.float() - ref).abs().max().item() < 2 ** -6 * ref.abs().max().item()
+    for name, lo in (("dq", 0), ("dk", H), ("dv", 2 * H)):
+        got, want = x.grad[:, lo:lo + H].float(), xr.grad[:, lo:lo + H]
+        e = (got - want).abs().max().item()
+        assert e < 2 ** -6 * want.abs().max().item(), f"{name} max err {e}"
+
+
 def test_attention_second_call_reuses_zeroed_scratch():
     B, S, nh, hd = 1, 256, 2, 128
     H = nh * hd
