@@ -176,8 +176,17 @@ __device__ __forceinline__ float block_absmax(float m, int lanes_per_block) {
 
 template <int BITS>
 __device__ __forceinline__ __half scale_from_absmax(float m) {
-  float s = __fdiv_rn(m, (float)Range<BITS>::qmax);
-  if (!(m > 0.0f)) s = 1.0f;
+  constexpr float q = (float)Range<BITS>::qmax;
+  float s;
+  if (__builtin_expect(m > 1.0e-30f && m < 3.0e38f, 1)) {
+    // the IEEE quotient by a constant from its correctly rounded reciprocal (see Divider)
+    constexpr float y = 1.0f / q;
+    const float q0 = __fmul_rn(m, y);
+    s = __fmaf_rn(__fmaf_rn(-q0, q, m), y, q0);
+  } else {
+    s = __fdiv_rn(m, q);
+    if (!(m > 0.0f)) s = 1.0f;
+  }
   return __float2half_rn(s);
 }
 
@@ -335,6 +344,10 @@ __device__ __forceinline__ Packed8<BITS> pack8(const int (&q)[GROUP]) {
 //     (lean_group_ok) and take the general path;
 //   * nearest rounding works on the SIGNED quotient (round-half-even is symmetric), so there is
 //     no |x| and no sign transfer;
+//   * stochastic rounding is a directed rounding: floor(n) + (u < frac(n)) is ceil(n - u), and with
+//     u = bits * 2^-16 the float f = 2^23 + bits (one byte permute of the hash) gives
+//     r = RU(n - f * 2^-16) = RU(n - u - 128), whose grid contains the integers, so that rounding
+//     r up to an integer (one more directed add) is ceil(n - u) - 128 exactly;
 //   * the clamped code c is turned into its stored form by ONE add, t = c + (1.5 * 2^23 - qmin):
 //     the float's bit pattern is 0x4B400000 + (c - qmin);
 //   * the bit pattern is multiplied into its place with an integer multiply-add; the constant
@@ -361,18 +374,22 @@ __device__ __forceinline__ Packed8<BITS> quant8_pack_lean(const float (&x)[GROUP
   constexpr uint32_t magic_bits = 0x4B400000u;                // bits of `magic` + (c - qmin)
   constexpr int PER_WORD = BITS == 8 ? 4 : 8;
   const float y = __frcp_rn(sf);
-  float u[GROUP];
+  float f[GROUP];  // 2^23 + the element's 16 random bits
   if constexpr (SR) {
     if ((idx0 & 1u) == 0u) {  // the usual case: two elements share one hash
 #pragma unroll
       for (int i = 0; i < GROUP; i += 2) {
-        const uint32_t h = sr_hash(key, (idx0 + i) >> 1);
-        u[i] = sr_u16(h & 0xFFFFu);
-        u[i + 1] = sr_u16(h >> 16);
+        const uint32_t h = sr_hash(key, (idx0 >> 1) + i / 2);
+        f[i] = __uint_as_float(__byte_perm(h, 0x4B000000u, 0x7410));
+        f[i + 1] = __uint_as_float(__byte_perm(h, 0x4B000000u, 0x7432));
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < GROUP; ++i) u[i] = sr_uniform(key, idx0 + i);
+      for (int i = 0; i < GROUP; ++i) {
+        const uint32_t h = sr_hash(key, (idx0 + i) >> 1);
+        f[i] = __uint_as_float(
+            __byte_perm(((idx0 + i) & 1u) ? h >> 16 : h, 0x4B000000u, 0x7410));
+      }
     }
   }
   Packed8<BITS> out;
@@ -385,9 +402,8 @@ __device__ __forceinline__ Packed8<BITS> quant8_pack_lean(const float (&x)[GROUP
       const float a = fabsf(x[i]);
       const float q0 = __fmul_rn(a, y);
       const float n = __fmaf_rn(__fmaf_rn(-q0, sf, a), y, q0);   // IEEE a / sf (see Divider)
-      const float fl = __fsub_rn(__fadd_rd(n, kTwo23), kTwo23);  // floor(n)
-      const float frac = __fsub_rn(n, fl);
-      const float mag = u[i] < frac ? __fadd_rn(fl, 1.0f) : fl;
+      const float r = __fmaf_ru(f[i], -0x1p-16f, n);
+      const float mag = __fsub_rn(__fadd_ru(r, kMagic), kMagic - 128.0f);
       s = BITS == 1 ? mag
                     : __uint_as_float(__float_as_uint(mag) | (__float_as_uint(x[i]) & 0x80000000u));
     } else {

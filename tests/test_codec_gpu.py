@@ -43,6 +43,32 @@ def test_blockwise_bit_exact(dtype, bits, block, n):
         assert d.dtype == out_dtype and torch.equal(d.cpu(), dc)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("bits", [1, 2, 4, 8])
+@pytest.mark.parametrize("block,tail", [(256, 0), (256, 16), (256, 9), (16, 1), (32, 250), (8, 5)])
+def test_large_tensors_bit_exact(dtype, bits, block, tail):
+    """From 1 Mi elements on a thread owns sixteen elements (two groups of a block, or the
+    one-group kernel at block 8): ragged tails, and every kind of block scale: zero, subnormal and
+    underflowing fp16 scales, overflow, NaN; nearest and stochastic at an odd offset."""
+    n = (1 << 20) + tail
+    g = torch.Generator().manual_seed(n + bits + block)
+    x = torch.randn(n, generator=g)
+    magnitude = torch.tensor([1e-2, 0.0, 2e-5, 3e-7, 1e-8, 5e4, 1e-38, 1.0])
+    x *= magnitude[(torch.arange(n) // block) % magnitude.numel()]
+    x[3 * 8 * block + 1], x[5 * 8 * block + 2], x[n - 1] = float("nan"), float("inf"), 7.0
+    x = x.to(dtype)
+    for kw in (dict(), dict(stochastic_rounding=True, sr_seed=11, sr_offset=12345),
+               dict(stochastic_rounding=True, sr_seed=12, sr_offset=2 ** 32 - 64)):
+        p, s, _ = Q.quantize_pack_tensor_blockwise(x.cuda(), bits, block_size=block, **kw)
+        pc, sc, _ = Q.quantize_pack_tensor_blockwise(x, bits, block_size=block, **kw)
+        assert torch.equal(s.cpu().view(torch.int16), sc.view(torch.int16))
+        assert torch.equal(p.cpu(), pc)
+    d = Q.unpack_dequantize_tensor_blockwise(p, s, bits, n, block_size=block, dtype=dtype)
+    dc = Q.unpack_dequantize_tensor_blockwise(pc, sc, bits, n, block_size=block, dtype=dtype)
+    assert torch.equal(torch.nan_to_num(d.cpu().float()), torch.nan_to_num(dc.float()))
+    assert torch.equal(d.cpu().isnan(), dc.isnan())
+
+
 def test_blockwise_unaligned_view_and_zero_blocks():
     x = torch.randn(5003)
     x[256:512] = 0
