@@ -27,6 +27,7 @@ def _get():
             lib.bcom_norm_bwd_scratch_elems.argtypes = [ci, ci]
             lib.bcom_norm_bwd_scratch_elems.restype = ll
             lib.bcom_rope.argtypes = [vp, vp, vp, ll, ci, ci, ll, ci, ci, vp]
+            lib.bcom_rope_copy.argtypes = [vp, vp, vp, vp, ll, ci, ci, ll, ci, ci, ci, vp]
             lib.bcom_layernorm_fwd.argtypes = [vp, vp, vp, vp, vp, vp, ci, ci, cf, vp]
             lib.bcom_layernorm_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, vp]
             lib.bcom_bias_gelu_fwd.argtypes = [vp, vp, vp, ll, ci, vp]
@@ -187,9 +188,8 @@ class RopeQKFunction(torch.autograd.Function):
     def forward(ctx, qkv, cos, sin, heads, head_dim, seq):
         ctx.mark_dirty(qkv)
         q2 = qkv.view(-1, qkv.shape[-1])
-        width = heads * head_dim
-        _rope_inplace(q2, 0, heads, head_dim, cos, sin, seq, False)
-        _rope_inplace(q2, width, heads, head_dim, cos, sin, seq, False)
+        # q and k are neighbours in a row: twice the heads in one pass
+        _rope_inplace(q2, 0, 2 * heads, head_dim, cos, sin, seq, False)
         ctx.save_for_backward(cos, sin)
         ctx.meta = (heads, head_dim, seq)
         return qkv
@@ -200,11 +200,17 @@ class RopeQKFunction(torch.autograd.Function):
         heads, head_dim, seq = ctx.meta
         d = dqkv.contiguous()
         if d.data_ptr() == dqkv.data_ptr():
+            if d.is_cuda and not torch.is_grad_enabled():
+                # the incoming gradient is not ours to change: rotate q and k, copy v, in one pass
+                out = torch.empty_like(d)
+                rows = d.view(-1, d.shape[-1])
+                check(_need().bcom_rope_copy(
+                    ptr(d), ptr(out), ptr(cos), ptr(sin), rows.shape[0], 2 * heads, head_dim,
+                    rows.shape[1], rows.shape[1], seq, 1, stream_ptr(d.device)), "rope_copy")
+                return out, None, None, None, None, None
             d = d.clone()
         d2 = d.view(-1, d.shape[-1])
-        width = heads * head_dim
-        _rope_inplace(d2, 0, heads, head_dim, cos, sin, seq, True)
-        _rope_inplace(d2, width, heads, head_dim, cos, sin, seq, True)
+        _rope_inplace(d2, 0, 2 * heads, head_dim, cos, sin, seq, True)
         return d, None, None, None, None, None
 
 
