@@ -30,12 +30,12 @@ __device__ __forceinline__ uint32_t epi_swz(int r, int u) {
 // 32), columns [n0, n0 + BN) are written where row < M and column < N (N % 8 == 0).
 // R (bf16 [M, N] with leading dimension ldr, or null): added to the product before the bf16
 // result is rounded (a linear layer whose output joins a residual stream: C = R + A x B in one
-// pass instead of a GEMM and an add kernel).
+// pass instead of a GEMM and an add kernel).  bias (bf16 [N], 16-byte aligned, or null): likewise.
 template <int BN, bool OUT_F32, bool ACCUM>
 __device__ __forceinline__ void store_accumulator_tma(uint32_t taddr, const CUtensorMap* tmC,
                                                       uint8_t* stage, int row0, int n0, int M,
                                                       int N, const void* R, long long ldr,
-                                                      int lane) {
+                                                      const void* bias, int lane) {
   static_assert(OUT_F32 || !ACCUM, "bf16 accumulation reads C: store_accumulator_rows");
   constexpr int COLS = OUT_F32 ? 32 : 64;
   if (row0 >= M) return;
@@ -75,6 +75,13 @@ __device__ __forceinline__ void store_accumulator_tma(uint32_t taddr, const CUte
         float f[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r[8 * u + i]);
+        if (bias != nullptr && col0 + u * 8 < N) {  // one address for the whole warp
+          const uint4 b = __ldg(reinterpret_cast<const uint4*>(
+              reinterpret_cast<const __nv_bfloat16*>(bias) + col0 + u * 8));
+          const __nv_bfloat16* bh = reinterpret_cast<const __nv_bfloat16*>(&b);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) f[i] += __bfloat162float(bh[i]);
+        }
         if (add && col0 + u * 8 < N) {
           const __nv_bfloat16* rh = reinterpret_cast<const __nv_bfloat16*>(&res[u]);
 #pragma unroll
@@ -133,11 +140,12 @@ template <int BN, bool OUT_F32, bool ACCUM>
 __device__ __forceinline__ void write_accumulator(uint32_t taddr, const CUtensorMap* tmC,
                                                   uint8_t* stage, void* C, long long ldc, int row0,
                                                   int n0, int M, int N, const void* R,
-                                                  long long ldr, int lane) {
+                                                  long long ldr, const void* bias, int lane) {
   if constexpr (!OUT_F32 && ACCUM)
     accumulate_bf16_rows<BN>(taddr, C, ldc, row0 + lane, n0, M, N);
   else
-    store_accumulator_tma<BN, OUT_F32, ACCUM>(taddr, tmC, stage, row0, n0, M, N, R, ldr, lane);
+    store_accumulator_tma<BN, OUT_F32, ACCUM>(taddr, tmC, stage, row0, n0, M, N, R, ldr, bias,
+                                              lane);
 }
 
 // Tensor map of C for the boxes above.

@@ -64,6 +64,7 @@ __device__ unsigned int g_status[4];
 struct Params {
   void* C;
   const void* R;  // optional bf16 residual added in the bf16 epilogue (see gemm_epilogue.cuh)
+  const void* bias;  // optional bf16 [N], likewise
   long long ldc, ldr;
   int M, N, K;
   int tiles_m, tiles_n;
@@ -241,11 +242,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int row0 = wi.m0 + quarter * 32;
       if (p.splits == 1)
         write_accumulator<BN, OUT_F32, ACCUM>(taddr, &tmC, epi + quarter * EPI_WARP_BYTES, p.C,
-                                              p.ldc, row0, wi.n0, p.M, p.N, p.R, p.ldr, lane);
+                                              p.ldc, row0, wi.n0, p.M, p.N, p.R, p.ldr, p.bias,
+                                              lane);
       else if constexpr (OUT_F32 && !ACCUM)
         write_accumulator<BN, true, false>(taddr, &tmC, epi + quarter * EPI_WARP_BYTES, p.C, p.ldc,
                                            wi.split * p.split_rows + row0, wi.n0,
-                                           p.splits * p.split_rows, p.N, nullptr, 0, lane);
+                                           p.splits * p.split_rows, p.N, nullptr, 0, nullptr, lane);
       tc::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&sh->acc_empty[buf]);
@@ -296,12 +298,13 @@ static Kernel pick(bool a_mn, bool b_mn, bool out_f32, bool accum) {
               : pick_out<BN, false, false>(out_f32, accum);
 }
 
-// C (bf16 or fp32) = sum over splits of the partial tiles, in ascending order (+ residual or + C).
+// C (bf16 or fp32) = sum over splits of the partial tiles, in ascending order (+ bias, + residual or + C).
 // Reads what the product kernel has just written (it is still in the L2).
 template <bool OUT_F32, bool ACCUM>
 __global__ void __launch_bounds__(256)
 split_sum_kernel(const float* __restrict__ ws, int splits, long long split_stride, void* C,
-                 const __nv_bfloat16* __restrict__ R, long long ldc, long long ldr, int M, int N) {
+                 const __nv_bfloat16* __restrict__ R, const __nv_bfloat16* __restrict__ bias,
+                 long long ldc, long long ldr, int M, int N) {
   const int vec = N / 4;
   const long long total = (long long)M * vec;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -325,6 +328,13 @@ split_sum_kernel(const float* __restrict__ ws, int splits, long long split_strid
       *dst = a;
     } else {
       __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(C) + row * ldc + col;
+      if (!ACCUM && bias) {
+        const uint2 o = *reinterpret_cast<const uint2*>(bias + col);
+        a.x += __uint_as_float(o.x << 16);
+        a.y += __uint_as_float(o.x & 0xffff0000u);
+        a.z += __uint_as_float(o.y << 16);
+        a.w += __uint_as_float(o.y & 0xffff0000u);
+      }
       const __nv_bfloat16* add = ACCUM ? dst : R ? R + row * ldr + col : nullptr;
       if (add) {
         const uint2 o = *reinterpret_cast<const uint2*>(add);
@@ -342,7 +352,8 @@ split_sum_kernel(const float* __restrict__ ws, int splits, long long split_strid
 
 // One launch of the product kernel; `splits` > 1: `C` is the fp32 workspace.
 template <int BN>
-static int launch(const void* A, const void* B, void* C, const void* residual, int M, int N, int K,
+static int launch(const void* A, const void* B, void* C, const void* residual, const void* bias,
+                  int M, int N, int K,
                   long long lda, long long ldb, long long ldc, long long ldr, bool a_mn, bool b_mn,
                   bool out_fp32, bool accumulate, int splits, int max_ctas, cudaStream_t stream) {
   CUtensorMap tmA, tmB, tmC;
@@ -352,6 +363,7 @@ static int launch(const void* A, const void* B, void* C, const void* residual, i
   Params p;
   p.C = C;
   p.R = residual;
+  p.bias = bias;
   p.ldc = ldc;
   p.ldr = ldr;
   p.M = M;
@@ -376,14 +388,15 @@ static int launch(const void* A, const void* B, void* C, const void* residual, i
   return (int)cudaGetLastError();
 }
 
-static int check_args(const void* A, const void* B, const void* C, const void* residual, int N,
-                      long long lda, long long ldb, long long ldc, long long ldr, bool out_fp32,
+static int check_args(const void* A, const void* B, const void* C, const void* residual,
+                      const void* bias, int N, long long lda, long long ldb, long long ldc, long long ldr, bool out_fp32,
                       bool accumulate) {
   // argument errors get codes of their own (1001..1008) so that they cannot be mistaken
   // for a CUDA error
   if ((lda % 8) || (ldb % 8) || (ldc % (out_fp32 ? 4 : 8)) || (N % 8)) return 1001;
   if (((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15)) return 1002;
   if (residual && (out_fp32 || accumulate || (ldr % 8) || ((uintptr_t)residual & 15))) return 1001;
+  if (bias && (out_fp32 || accumulate || ((uintptr_t)bias & 15))) return 1001;
   return 0;
 }
 
@@ -398,19 +411,28 @@ extern "C" {
 // Leading dimensions are in elements and must keep rows 16-byte aligned.
 //   residual (optional, bf16 [M, N], leading dimension ldr): C = residual + A x B; only with a
 //   bf16, non-accumulating C
+//   bias (optional, bf16 [N], 16-byte aligned): added to every row; same condition
+int bcom_gemm_bf16_bias(const void* A, const void* B, void* C, const void* residual,
+                        const void* bias, int M, int N, int K, long long lda, long long ldb,
+                        long long ldc, long long ldr, int a_mn_major, int b_mn_major, int out_fp32,
+                        int accumulate, int max_ctas, void* stream) {
+  using namespace gemm;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (const int rc = check_args(A, B, C, residual, bias, N, lda, ldb, ldc, ldr, out_fp32 != 0,
+                                accumulate != 0))
+    return rc;
+  (void)cudaGetLastError();  // do not inherit an error left behind by an earlier call
+  return launch<256>(A, B, C, residual, bias, M, N, K, lda, ldb, ldc, ldr, a_mn_major != 0,
+                     b_mn_major != 0, out_fp32 != 0, accumulate != 0, 1, max_ctas,
+                     (cudaStream_t)stream);
+}
+
 int bcom_gemm_bf16_ex(const void* A, const void* B, void* C, const void* residual, int M, int N,
                       int K, long long lda, long long ldb, long long ldc, long long ldr,
                       int a_mn_major, int b_mn_major, int out_fp32, int accumulate, int max_ctas,
                       void* stream) {
-  using namespace gemm;
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (const int rc = check_args(A, B, C, residual, N, lda, ldb, ldc, ldr, out_fp32 != 0,
-                                accumulate != 0))
-    return rc;
-  (void)cudaGetLastError();  // do not inherit an error left behind by an earlier call
-  return launch<256>(A, B, C, residual, M, N, K, lda, ldb, ldc, ldr, a_mn_major != 0,
-                     b_mn_major != 0, out_fp32 != 0, accumulate != 0, 1, max_ctas,
-                     (cudaStream_t)stream);
+  return bcom_gemm_bf16_bias(A, B, C, residual, nullptr, M, N, K, lda, ldb, ldc, ldr, a_mn_major,
+                             b_mn_major, out_fp32, accumulate, max_ctas, stream);
 }
 
 // fp32 elements of workspace that bcom_gemm_bf16_split needs (0 for splits <= 1)
@@ -423,23 +445,23 @@ long long bcom_gemm_split_workspace(int M, int N, int splits) {
 // i.e. 16 of 148 SMs fetching the weights in 64 serial k-blocks each.  splits > 1: the partial
 // tiles go to `workspace` (private to the call until it has run, 16-byte aligned) and a second
 // kernel adds them up in ascending order.  `splits` must not exceed the 64-wide k-blocks.
-int bcom_gemm_bf16_split(const void* A, const void* B, void* C, const void* residual, int M, int N,
-                         int K, long long lda, long long ldb, long long ldc, long long ldr,
+int bcom_gemm_bf16_split(const void* A, const void* B, void* C, const void* residual,
+                         const void* bias, int M, int N, int K, long long lda, long long ldb, long long ldc, long long ldr,
                          int a_mn_major, int b_mn_major, int out_fp32, int accumulate, int splits,
                          void* workspace, void* stream) {
   using namespace gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (const int rc = check_args(A, B, C, residual, N, lda, ldb, ldc, ldr, out_fp32 != 0,
+  if (const int rc = check_args(A, B, C, residual, bias, N, lda, ldb, ldc, ldr, out_fp32 != 0,
                                 accumulate != 0))
     return rc;
   if (splits < 1 || splits > 8 || splits > (K + BK - 1) / BK) return (int)cudaErrorInvalidValue;
   (void)cudaGetLastError();
   cudaStream_t st = (cudaStream_t)stream;
   if (splits == 1)
-    return launch<128>(A, B, C, residual, M, N, K, lda, ldb, ldc, ldr, a_mn_major != 0,
+    return launch<128>(A, B, C, residual, bias, M, N, K, lda, ldb, ldc, ldr, a_mn_major != 0,
                        b_mn_major != 0, out_fp32 != 0, accumulate != 0, 1, 0, st);
   if (!workspace || ((uintptr_t)workspace & 15)) return 1002;
-  const int rc = launch<128>(A, B, workspace, nullptr, M, N, K, lda, ldb, N, 0, a_mn_major != 0,
+  const int rc = launch<128>(A, B, workspace, nullptr, nullptr, M, N, K, lda, ldb, N, 0, a_mn_major != 0,
                              b_mn_major != 0, true, false, splits, 0, st);
   if (rc) return rc;
   const long long stride = (long long)((M + BM - 1) / BM * BM) * N;
@@ -447,16 +469,21 @@ int bcom_gemm_bf16_split(const void* A, const void* B, void* C, const void* resi
   const int grid = (int)(work < 4LL * sm_count() ? work : 4LL * sm_count());
   const float* ws = (const float*)workspace;
   const __nv_bfloat16* R = (const __nv_bfloat16*)residual;
+  const __nv_bfloat16* b = (const __nv_bfloat16*)bias;
   if (out_fp32) {
     if (accumulate)
-      split_sum_kernel<true, true><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, ldc, ldr, M, N);
+      split_sum_kernel<true, true><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, b, ldc, ldr, M,
+                                                        N);
     else
-      split_sum_kernel<true, false><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, ldc, ldr, M, N);
+      split_sum_kernel<true, false><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, b, ldc, ldr, M,
+                                                        N);
   } else {
     if (accumulate)
-      split_sum_kernel<false, true><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, ldc, ldr, M, N);
+      split_sum_kernel<false, true><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, b, ldc, ldr, M,
+                                                        N);
     else
-      split_sum_kernel<false, false><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, ldc, ldr, M, N);
+      split_sum_kernel<false, false><<<grid, 256, 0, st>>>(ws, splits, stride, C, R, b, ldc, ldr, M,
+                                                        N);
   }
   return (int)cudaGetLastError();
 }

@@ -65,6 +65,7 @@ __device__ unsigned long long* g_profile;
 struct Params {
   void* C;
   const void* R;  // optional bf16 residual added in the bf16 epilogue
+  const void* bias;  // optional bf16 [N], likewise
   long long ldc, ldr;
   int M, N, K;
   int tiles_m, tiles_n;
@@ -352,7 +353,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       const uint32_t taddr = tmem_base + (uint32_t)buf * BN + ((uint32_t)(quarter * 32) << 16);
       gemm::write_accumulator<BN, OUT_F32, ACCUM>(
           taddr, &tmC, epi + quarter * gemm::EPI_WARP_BYTES, p.C, p.ldc,
-          tm * BM + (int)rank * BM_CTA + quarter * 32, tn * BN, p.M, p.N, p.R, p.ldr, lane);
+          tm * BM + (int)rank * BM_CTA + quarter * 32, tn * BN, p.M, p.N, p.R, p.ldr, p.bias, lane);
       tc::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
@@ -435,15 +436,16 @@ extern "C" {
 
 
 // Same contract as bcom_gemm_bf16 (gemm_tcgen05.cu); max_ctas counts CTAs (two per pair).
-int bcom_gemm2_bf16_ex(const void* A, const void* B, void* C, const void* residual, int M, int N,
-                       int K, long long lda, long long ldb, long long ldc, long long ldr,
-                       int a_mn_major, int b_mn_major, int out_fp32, int accumulate,
-                       int max_ctas, void* stream) {
+int bcom_gemm2_bf16_bias(const void* A, const void* B, void* C, const void* residual,
+                         const void* bias, int M, int N, int K, long long lda, long long ldb,
+                         long long ldc, long long ldr, int a_mn_major, int b_mn_major,
+                         int out_fp32, int accumulate, int max_ctas, void* stream) {
   using namespace gemm2;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda % 8) || (ldb % 8) || (ldc % (out_fp32 ? 4 : 8)) || (N % 8)) return 1001;
   if (((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15)) return 1002;
   if (residual && (out_fp32 || accumulate || (ldr % 8) || ((uintptr_t)residual & 15))) return 1001;
+  if (bias && (out_fp32 || accumulate || ((uintptr_t)bias & 15))) return 1001;
   (void)cudaGetLastError();
   CUtensorMap tmA, tmB, tmC;
   tc::bind_context_once();
@@ -457,6 +459,7 @@ int bcom_gemm2_bf16_ex(const void* A, const void* B, void* C, const void* residu
   Params p;
   p.C = C;
   p.R = residual;
+  p.bias = bias;
   p.ldc = ldc;
   p.ldr = ldr;
   p.M = M;
@@ -473,6 +476,14 @@ int bcom_gemm2_bf16_ex(const void* A, const void* B, void* C, const void* residu
   if (pairs < 1) pairs = 1;
   kernel<<<2 * pairs, kThreads, SMEM_BYTES, (cudaStream_t)stream>>>(tmA, tmB, tmC, p);
   return (int)cudaGetLastError();
+}
+
+int bcom_gemm2_bf16_ex(const void* A, const void* B, void* C, const void* residual, int M, int N,
+                       int K, long long lda, long long ldb, long long ldc, long long ldr,
+                       int a_mn_major, int b_mn_major, int out_fp32, int accumulate,
+                       int max_ctas, void* stream) {
+  return bcom_gemm2_bf16_bias(A, B, C, residual, nullptr, M, N, K, lda, ldb, ldc, ldr, a_mn_major,
+                              b_mn_major, out_fp32, accumulate, max_ctas, stream);
 }
 
 int bcom_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,

@@ -106,7 +106,8 @@ class GPT2(torch.nn.Module):
                 # the layer's own parameters has been produced by then
                 x.register_hook(self._make_hook(i))
             h = ln(x, self._w(f"h{i}.ln1_w"), self._w(f"h{i}.ln1_b"))
-            qkv = G.linear(h, self._w(f"h{i}.wqkv")) + self._w(f"h{i}.bqkv")
+            # biases and residual sums live in the GEMM epilogues
+            qkv = G.linear(h, self._w(f"h{i}.wqkv"), bias=self._w(f"h{i}.bqkv"))
             if fused_attn:
                 a = A.attention(qkv, B, S, nh, hd)
             else:
@@ -114,10 +115,10 @@ class GPT2(torch.nn.Module):
                            for j in range(3))
                 a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
                 a = a.transpose(1, 2).reshape(B * S, D)
-            x = x + G.linear(a, self._w(f"h{i}.wo")) + self._w(f"h{i}.bo")
+            x = G.linear(a, self._w(f"h{i}.wo"), residual=x, bias=self._w(f"h{i}.bo"))
             h = ln(x, self._w(f"h{i}.ln2_w"), self._w(f"h{i}.ln2_b"))
             h = gelu(G.linear(h, self._w(f"h{i}.wfc")), self._w(f"h{i}.bfc"))
-            x = x + G.linear(h, self._w(f"h{i}.wproj")) + self._w(f"h{i}.bproj")
+            x = G.linear(h, self._w(f"h{i}.wproj"), residual=x, bias=self._w(f"h{i}.bproj"))
         x = ln(x, self._w("lnf_w"), self._w("lnf_b"))
         logits = G.linear(x, self._w("wte"))
         if targets is None:

@@ -32,7 +32,11 @@ def _get():
                                            ci, vp]
             lib.bcom_gemm_bf16_ex.argtypes = [vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci, ci,
                                               ci, ci, ci, vp]
-            lib.bcom_gemm_bf16_split.argtypes = [vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci,
+            lib.bcom_gemm_bf16_bias.argtypes = [vp, vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci,
+                                                ci, ci, ci, ci, vp]
+            lib.bcom_colsum_bf16.argtypes = [vp, vp, vp, ll, ci, vp]
+            lib.bcom_colsum_strips.argtypes = [ll, ci]
+            lib.bcom_gemm_bf16_split.argtypes = [vp, vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci,
                                                  ci, ci, ci, ci, vp, vp]
             lib.bcom_gemm_split_workspace.argtypes = [ci, ci, ci]
             lib.bcom_gemm_split_workspace.restype = ll
@@ -56,6 +60,8 @@ def _get2():
                                             ci, vp]
             lib.bcom_gemm2_bf16_ex.argtypes = [vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci,
                                                ci, ci, ci, ci, vp]
+            lib.bcom_gemm2_bf16_bias.argtypes = [vp, vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci,
+                                                 ci, ci, ci, ci, vp]
             lib.bcom_gemm2_status.argtypes = [ctypes.POINTER(ctypes.c_uint * 4), ci]
             lib.bcom_gemm2_set_profile.argtypes = [vp]
         _lib2 = lib if lib is not None else False
@@ -165,10 +171,13 @@ def use_library_gemm(on: bool) -> bool:
     return old
 
 
-def _gemm_library(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residual=None):
+def _gemm_library(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residual=None,
+                  bias=None):
     A = a.t() if a_mn_major else a
     B = b if b_mn_major else b.t()
     c = torch.matmul(A, B)
+    if bias is not None:
+        c = c + bias
     if residual is not None:
         c = c + residual
     if out is None:
@@ -180,7 +189,8 @@ def _gemm_library(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, resi
     return out
 
 
-def _gemm_host(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residual=None):
+def _gemm_host(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residual=None,
+               bias=None):
     """The kernel's contract for tensors that live on the CPU (fp32 accumulation, result
     rounded once): CPU ranks run the trainers' plumbing with it."""
     A = a.float().t() if a_mn_major else a.float()
@@ -188,6 +198,8 @@ def _gemm_host(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residua
     if A.shape[1] != B.shape[0]:
         raise ValueError(f"reduction dimensions differ: {A.shape[1]} vs {B.shape[0]}")
     c = A @ B
+    if bias is not None:
+        c = c + bias.float()
     if residual is not None:
         c = c + residual.float()
     if out is None:
@@ -203,22 +215,25 @@ def _gemm_host(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residua
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False,
          b_mn_major: bool = False, out: Optional[torch.Tensor] = None,
          out_dtype: torch.dtype = torch.bfloat16, accumulate: bool = False,
-         max_ctas: int = 0, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+         max_ctas: int = 0, residual: Optional[torch.Tensor] = None,
+         bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``C[M, N] (+)= A x B`` with bf16 operands and fp32 accumulation.
 
     ``a``: ``[M, K]`` (K-major) or, with ``a_mn_major``, stored ``[K, M]``.
     ``b``: ``[N, K]`` (K-major) or, with ``b_mn_major``, stored ``[K, N]``.
     Operands are 2-D with unit stride in the last dimension; row strides are free.
     ``residual`` (bf16 ``[M, N]``, bf16 non-accumulating output only): ``C = residual + A x B``,
-    added in the epilogue before the result is rounded.
+    added in the epilogue before the result is rounded.  ``bias`` (bf16 ``[N]``, contiguous and
+    16-byte aligned): added to every row in the same place, under the same condition.
     """
-    if residual is not None and (accumulate or (out is not None and out.dtype != torch.bfloat16)
+    if (residual is not None or bias is not None) and (accumulate or (out is not None and out.dtype != torch.bfloat16)
                                  or (out is None and out_dtype != torch.bfloat16)):
-        raise ValueError("residual needs a bf16, non-accumulating output")
+        raise ValueError("residual and bias need a bf16, non-accumulating output")
     if not a.is_cuda:
-        return _gemm_host(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residual)
+        return _gemm_host(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residual, bias)
     if _library:
-        return _gemm_library(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residual)
+        return _gemm_library(a, b, a_mn_major, b_mn_major, out, out_dtype, accumulate, residual,
+                             bias)
     lib = _get()
     if lib is None:
         raise NativeError("tcgen05 GEMM needs the bcom_llama library and a GPU")
@@ -240,6 +255,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False,
     if residual is not None and (residual.shape != (M, N) or residual.stride(1) != 1
                                  or residual.dtype != torch.bfloat16):
         raise ValueError("bad residual tensor")
+    if bias is not None and (bias.shape != (N,) or bias.dtype != torch.bfloat16
+                             or not bias.is_contiguous()):
+        raise ValueError("bad bias tensor")
     kind = variant()
     plan = _plan(M, N, K, a_mn_major, max_ctas) if kind == "auto" else 0 if kind == "1cta" else -1
     with _native.on_device(a.device):
@@ -249,18 +267,38 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False,
                 ws = torch.empty(lib.bcom_gemm_split_workspace(M, N, plan), dtype=torch.float32,
                                  device=a.device)
             check(lib.bcom_gemm_bf16_split(
-                ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K, a.stride(0), b.stride(0),
+                ptr(a), ptr(b), ptr(out), ptr(residual), ptr(bias), M, N, K, a.stride(0), b.stride(0),
                 out.stride(0), 0 if residual is None else residual.stride(0), int(a_mn_major),
                 int(b_mn_major), int(out.dtype == torch.float32), int(accumulate), plan, ptr(ws),
                 stream_ptr(a.device)), "bcom_gemm_bf16_split", launches=1 + (plan > 1))
             return out
-        launch = lib.bcom_gemm_bf16_ex if plan == 0 else _get2().bcom_gemm2_bf16_ex
+        launch = lib.bcom_gemm_bf16_bias if plan == 0 else _get2().bcom_gemm2_bf16_bias
         check(launch(
-            ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K, a.stride(0), b.stride(0),
+            ptr(a), ptr(b), ptr(out), ptr(residual), ptr(bias), M, N, K, a.stride(0), b.stride(0),
             out.stride(0), 0 if residual is None else residual.stride(0),
             int(a_mn_major), int(b_mn_major), int(out.dtype == torch.float32),
             int(accumulate), int(max_ctas), stream_ptr(a.device)), "bcom_gemm_bf16")
     return out
+
+
+def _bias_grad(dy2: torch.Tensor, bias: torch.Tensor) -> Optional[torch.Tensor]:
+    """Column sums of ``dy2 [T, out]`` in fp32, into ``bias.main_grad`` where the parameter has
+    it (autograd then gets ``None``)."""
+    main = getattr(bias, "main_grad", None)
+    if not dy2.is_cuda:
+        s = dy2.float().sum(0)
+        if main is None:
+            return s.to(bias.dtype)
+        main.add_(s)
+        return None
+    rows, n = dy2.shape
+    lib = _get()
+    out = main if main is not None else torch.zeros(n, dtype=torch.float32, device=dy2.device)
+    partials = torch.empty(lib.bcom_colsum_strips(rows, n) * n, dtype=torch.float32,
+                           device=dy2.device)
+    check(lib.bcom_colsum_bf16(ptr(dy2), ptr(out), ptr(partials), rows, n,
+                               stream_ptr(dy2.device)), "colsum_bf16", launches=2)
+    return None if main is not None else out.to(bias.dtype)
 
 
 class LinearFunction(torch.autograd.Function):
@@ -272,10 +310,11 @@ class LinearFunction(torch.autograd.Function):
     """
 
     @staticmethod
-    def forward(ctx, x, weight, residual=None):
+    def forward(ctx, x, weight, residual=None, bias=None):
         """``residual`` (same shape as the output): ``y = residual + x W^T`` in the GEMM's
-        epilogue; its gradient is the output gradient itself."""
-        ctx.save_for_backward(x, weight)
+        epilogue; its gradient is the output gradient itself.  ``bias`` ``[out]``: added in the
+        same place; its gradient is accumulated like the weight's."""
+        ctx.save_for_backward(x, weight, bias)
         ctx.has_residual = residual is not None
         x2 = x.reshape(-1, x.shape[-1])
         # allocate with the final shape: the result must not be a view, later kernels
@@ -286,12 +325,13 @@ class LinearFunction(torch.autograd.Function):
             res2 = residual.reshape(-1, weight.shape[0])
             if res2.stride(-1) != 1:
                 res2 = res2.contiguous()
-        gemm(x2, weight, out=y.view(-1, weight.shape[0]), residual=res2)
+        extra = {} if bias is None else {"bias": bias}
+        gemm(x2, weight, out=y.view(-1, weight.shape[0]), residual=res2, **extra)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, weight = ctx.saved_tensors
+        x, weight, bias = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
@@ -315,10 +355,14 @@ class LinearFunction(torch.autograd.Function):
                 dw = None
             else:
                 dw = gemm(dy2, x2, a_mn_major=True, b_mn_major=True)
-        return dx, dw, (dy if ctx.has_residual and ctx.needs_input_grad[2] else None)
+        db = None
+        if bias is not None and ctx.needs_input_grad[3]:
+            db = _bias_grad(dy2, bias)
+        return dx, dw, (dy if ctx.has_residual and ctx.needs_input_grad[2] else None), db
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor,
-           residual: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``x W^T`` (``+ residual``, added inside the GEMM) on the tcgen05 kernels."""
-    return LinearFunction.apply(x, weight, residual)
+           residual: Optional[torch.Tensor] = None,
+           bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``x W^T`` (``+ residual``, ``+ bias``, added inside the GEMM) on the tcgen05 kernels."""
+    return LinearFunction.apply(x, weight, residual, bias)

@@ -41,9 +41,9 @@ MODULES = [
 ENVIRONMENT = [
     "## Environment variables", "",
     "| variable | effect |", "|---|---|",
-    "| `BITSCOM_GEMM` | `1cta` (default) or `2cta`: the kernel `ops.gemm.gemm` launches |",
+    "| `BITSCOM_GEMM` | `auto` (default, by shape), `1cta` or `2cta`: the kernel `ops.gemm.gemm` launches |",
     "| `BITSCOM_ATTN_FWD`, `BITSCOM_ATTN_BWD_DQ` | attention kernel variants (`simple` / "
-    "`pipelined`; `atomic` / `tma`) |",
+    "`pipelined` / `dual`; `atomic` / `tma` / `pipelined`) |",
     "| `BITSCOM_NVLS` | `1`: the all-gather half of the fused collective goes out as "
     "`multimem.st` through an NVLink multicast mapping (needs torch symmetric memory); "
     "default off |",

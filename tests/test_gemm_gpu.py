@@ -178,6 +178,47 @@ def test_gemm_split_k(monkeypatch, splits, a_mn, b_mn, M, N, K):
     G.check_status()
 
 
+@pytest.mark.parametrize("plan", [-1, 0, 1, 3])
+@pytest.mark.parametrize("M,N,K", [(200, 264, 520), (8, 8, 256), (384, 72, 1024)])
+def test_bias_in_the_epilogue(monkeypatch, plan, M, N, K):
+    """C = A B + bias (+ residual), each kernel, ragged edges; exact on small integers (one rounding
+    to bf16).  Accumulating or fp32 outputs refuse a bias."""
+    if plan < 0 and not G.pair_available():
+        pytest.skip("the CTA-pair library is not part of this installation")
+    monkeypatch.setattr(G, "_plan", lambda *a: plan)
+    a = torch.randint(-3, 4, (M, K), device="cuda").to(torch.bfloat16)
+    b = torch.randint(-3, 4, (N, K), device="cuda").to(torch.bfloat16)
+    bias = torch.randint(-9, 10, (N,), device="cuda").to(torch.bfloat16)
+    res = torch.randint(-9, 10, (M, N), device="cuda").to(torch.bfloat16)
+    ref = a.float() @ b.float().t() + bias.float()
+    assert torch.equal(G.gemm(a, b, bias=bias), ref.to(torch.bfloat16))
+    assert torch.equal(G.gemm(a, b, bias=bias, residual=res), (ref + res.float()).to(torch.bfloat16))
+    G.check_status()
+    with pytest.raises(ValueError):
+        G.gemm(a, b, bias=bias, out_dtype=torch.float32)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 8), (77, 264), (5000, 1032)])
+@pytest.mark.parametrize("main", [False, True])
+def test_linear_bias_gradient(rows, n, main):
+    x = _mk(rows, 64, 21).requires_grad_()
+    w = _mk(n, 64, 22).requires_grad_()
+    b = _mk(1, n, 23)[0].clone().requires_grad_()
+    dy = _mk(rows, n, 24)
+    if main:
+        b.main_grad = torch.ones(n, device="cuda")
+    y = G.linear(x, w, bias=b)
+    _check(y, x.detach().float() @ w.detach().float().t() + b.detach().float(), 64)
+    y.backward(dy)
+    want = dy.double().sum(0)
+    # fp32 sums of `rows` values below 3: rows * 2^-24 relative of their magnitudes' sum
+    bound = dy.double().abs().sum(0) * rows * 2.0 ** -24 + 1e-6
+    if main:
+        assert b.grad is None and ((b.main_grad.double() - 1 - want).abs() <= bound + 1e-5).all()
+    else:
+        assert torch.allclose(b.grad.double(), want, rtol=2 ** -8, atol=1e-2)
+
+
 def test_gemm_throughput_report():
     M = N = K = 8192
     a, b = _mk(M, K, 1), _mk(N, K, 2)
