@@ -400,7 +400,9 @@ class CrossEntropyFunction(torch.autograd.Function):
         lib = _need()
         rows, stream = l2.shape[0], stream_ptr(logits.device)
         per_row = torch.empty(rows, dtype=torch.float32, device=logits.device)
-        loss, valid, scale = torch.empty(3, dtype=torch.float32, device=logits.device).unbind()
+        # tensors of their own: a caller may change the loss in place, which views of one would refuse
+        loss, valid, scale = (torch.empty((), dtype=torch.float32, device=logits.device)
+                              for _ in range(3))
         # target count and scale, the rows, their sum: three launches
         check(lib.bcom_cross_entropy_scale(ptr(t), rows, int(ignore_index), float(loss_scale),
                                            ptr(valid), ptr(scale), stream), "cross_entropy_scale")
