@@ -22,3 +22,25 @@ def test_work_items_partition_the_output(tmp_path):
     run = subprocess.run([exe], capture_output=True, text=True, timeout=600)
     assert run.returncode == 0, run.stderr[-2000:]
     assert run.stdout.startswith("ok:")
+
+
+def test_plan_of_every_shape_can_be_launched():
+    """The rule that picks a kernel by shape: a share of K never exceeds the k-blocks, the
+    workspace of shared-out products stays small, and a capped grid never takes them."""
+    import random
+
+    from bitscom_b200.ops import gemm as G
+
+    rng = random.Random(5)
+    for _ in range(2000):
+        M, N, K = (rng.choice([1, 7, 64, 77, 128, 200, 577, 1000, 4096, 8192, 50432])
+                   for _ in range(3))
+        N = -(-N // 8) * 8
+        for a_mn in (False, True):
+            plan = G._plan(M, N, K, a_mn)
+            assert -1 <= plan <= 8
+            if plan >= 1:
+                assert plan <= -(-K // 64)
+                assert plan * -(-M // 128) * 128 * N * 4 <= 80 << 20 or plan == 1
+            assert G._plan(M, N, K, a_mn, 1) == 0
+            assert G._plan(M, N, K, a_mn, 64) in (-1, 0)
