@@ -126,7 +126,7 @@ def _plan(M: int, N: int, K: int, a_mn_major: bool = False, max_ctas: int = 0) -
         c = -(-small * splits // _SMS) * -(-kb // splits)
         return c + (16 + 4.9e-6 * splits * rows * 128 * N if splits > 1 else 0)
 
-    best = min(range(1, min(8, kb) + 1), key=cost)
+    best = min(range(1, min(8, max(kb, 1)) + 1), key=cost)
     return best if cost(best) < 1.33 * kb else 0
 
 

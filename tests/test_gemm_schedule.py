@@ -31,6 +31,8 @@ def test_plan_of_every_shape_can_be_launched():
 
     from bitscom_b200.ops import gemm as G
 
+    for empty in ((0, 8, 64), (8, 0, 64), (8, 8, 0)):  # nothing to do, but not refused
+        assert G._plan(*empty) >= 0
     rng = random.Random(5)
     for _ in range(2000):
         M, N, K = (rng.choice([1, 7, 64, 77, 128, 200, 577, 1000, 4096, 8192, 50432])
