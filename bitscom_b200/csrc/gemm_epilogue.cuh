@@ -6,13 +6,15 @@
 // The rows leave through shared memory: each thread writes its row of a 128-byte wide chunk
 // (64 bf16 or 32 fp32 columns, 128-byte swizzle: no bank conflicts), one lane sends the 32 x 128
 // byte box with a bulk tensor store, which also clips it at the edges of C.  Two chunks per
-// warp alternate, so the next one is read from tensor memory while the last one is on its way.
+// warp alternate over all its tiles, so the next one is read from tensor memory while the last
+// one is on its way.
 // An accumulating fp32 C (weight gradients) takes the box as a bulk reduction: the addition is
 // done by the L2, C is never read into an SM.  Stores straight from the registers, 16 bytes per
 // lane at a row's distance, cost 32 wavefronts per instruction and the accumulating form waited
 // on its reads (a gradient of 32000 x 4096 from 128 tokens took 350 us for 1 GB of traffic).
 #pragma once
 
+#include "gemm_schedule.cuh"
 #include "tc_common.cuh"
 
 namespace gemm {
@@ -35,7 +37,8 @@ template <int BN, bool OUT_F32, bool ACCUM>
 __device__ __forceinline__ void store_accumulator_tma(uint32_t taddr, const CUtensorMap* tmC,
                                                       uint8_t* stage, int row0, int n0, int M,
                                                       int N, const void* R, long long ldr,
-                                                      const void* bias, int lane) {
+                                                      const void* bias, int lane,
+                                                      gemm_sched::StagingChunks& chunks) {
   static_assert(OUT_F32 || !ACCUM, "bf16 accumulation reads C: store_accumulator_rows");
   constexpr int COLS = OUT_F32 ? 32 : 64;
   if (row0 >= M) return;
@@ -43,7 +46,7 @@ __device__ __forceinline__ void store_accumulator_tma(uint32_t taddr, const CUte
   for (int c = 0; c < BN / COLS; ++c) {
     const int col0 = n0 + c * COLS;
     if (col0 >= N) break;
-    uint8_t* buf = stage + (c & 1) * EPI_CHUNK_BYTES;
+    uint8_t* buf = stage + chunks.next() * EPI_CHUNK_BYTES;
     if constexpr (OUT_F32) {
       uint32_t r[32];
       tc::tmem_ld_32x32(taddr + c * COLS, r);
@@ -140,12 +143,13 @@ template <int BN, bool OUT_F32, bool ACCUM>
 __device__ __forceinline__ void write_accumulator(uint32_t taddr, const CUtensorMap* tmC,
                                                   uint8_t* stage, void* C, long long ldc, int row0,
                                                   int n0, int M, int N, const void* R,
-                                                  long long ldr, const void* bias, int lane) {
+                                                  long long ldr, const void* bias, int lane,
+                                                  gemm_sched::StagingChunks& chunks) {
   if constexpr (!OUT_F32 && ACCUM)
     accumulate_bf16_rows<BN>(taddr, C, ldc, row0 + lane, n0, M, N);
   else
     store_accumulator_tma<BN, OUT_F32, ACCUM>(taddr, tmC, stage, row0, n0, M, N, R, ldr, bias,
-                                              lane);
+                                              lane, chunks);
 }
 
 // Tensor map of C for the boxes above.

@@ -36,4 +36,14 @@ __host__ __device__ inline int split_begin(int num_kb, int splits, int split) {
   return (int)((long long)num_kb * split / splits);
 }
 
+// Which of its two staging chunks an epilogue warp fills next.  It waits for all of its bulk stores
+// but the newest one before it fills a chunk, so the chunk must never be the one that the newest
+// store reads: the two alternate over everything the warp sends.  A tile whose last columns are an
+// odd number of chunks must not make the next tile start with the same one again, hence a counter
+// that lives as long as the warp and not the tile.
+struct StagingChunks {
+  unsigned sent = 0;
+  __host__ __device__ int next() { return (int)(sent++ & 1u); }
+};
+
 }  // namespace gemm_sched

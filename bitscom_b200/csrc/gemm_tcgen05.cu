@@ -228,6 +228,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else {
     // ------------------------------ epilogue -----------------------------------
     const int quarter = warp & 3;  // TMEM lanes this warp may read: 32*quarter ..
+    gemm_sched::StagingChunks chunks;
     int iter = 0;
     for (int t = blockIdx.x; t < total_tiles && !sh->abort; t += gridDim.x, ++iter) {
       const WorkItem wi = work_item<BN>(p, t);
@@ -243,11 +244,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (p.splits == 1)
         write_accumulator<BN, OUT_F32, ACCUM>(taddr, &tmC, epi + quarter * EPI_WARP_BYTES, p.C,
                                               p.ldc, row0, wi.n0, p.M, p.N, p.R, p.ldr, p.bias,
-                                              lane);
+                                              lane, chunks);
       else if constexpr (OUT_F32 && !ACCUM)
         write_accumulator<BN, true, false>(taddr, &tmC, epi + quarter * EPI_WARP_BYTES, p.C, p.ldc,
                                            wi.split * p.split_rows + row0, wi.n0,
-                                           p.splits * p.split_rows, p.N, nullptr, 0, nullptr, lane);
+                                           p.splits * p.split_rows, p.N, nullptr, 0, nullptr, lane,
+                                           chunks);
       tc::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&sh->acc_empty[buf]);

@@ -339,6 +339,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
   } else {
     // ------------------------------ epilogue (both CTAs) -------------------------
     const int quarter = warp & 3;  // TMEM lanes this warp may read: 32*quarter ..
+    gemm_sched::StagingChunks chunks;
     int iter = 0;
     for (int t = pair; t < total_tiles && !sh->abort; t += num_pairs, ++iter) {
       int tm, tn;
@@ -353,7 +354,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA,
       const uint32_t taddr = tmem_base + (uint32_t)buf * BN + ((uint32_t)(quarter * 32) << 16);
       gemm::write_accumulator<BN, OUT_F32, ACCUM>(
           taddr, &tmC, epi + quarter * gemm::EPI_WARP_BYTES, p.C, p.ldc,
-          tm * BM + (int)rank * BM_CTA + quarter * 32, tn * BN, p.M, p.N, p.R, p.ldr, p.bias, lane);
+          tm * BM + (int)rank * BM_CTA + quarter * 32, tn * BN, p.M, p.N, p.R, p.ldr, p.bias, lane,
+          chunks);
       tc::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {

@@ -27,6 +27,28 @@ static int check(int M, int N) {
   return 0;
 }
 
+// The staging chunks of an epilogue warp.  It waits until at most its newest store is under way
+// and then fills a chunk, while that store may still be reading another: over the tiles that each
+// of `ctas` CTAs takes, no two stores in a row may use the same chunk.  `cols`: columns per chunk
+// (64 bf16, 32 fp32).
+template <int BN>
+static int check_staging(int M, int N, int ctas, int cols) {
+  const int tiles_m = (M + 127) / 128, tiles_n = (N + BN - 1) / BN;
+  for (int cta = 0; cta < ctas; ++cta) {
+    gemm_sched::StagingChunks chunks;
+    int newest = -1;  // chunk that the newest store reads
+    for (int w = cta; w < tiles_m * tiles_n; w += ctas) {
+      const gemm_sched::WorkItem wi = gemm_sched::work_item<128, BN, 8>(tiles_m, tiles_n, w);
+      for (int c = 0; c < BN / cols && wi.n0 + c * cols < N; ++c) {
+        const int chunk = chunks.next();
+        if (chunk < 0 || chunk > 1 || chunk == newest) return 10;
+        newest = chunk;
+      }
+    }
+  }
+  return 0;
+}
+
 int main() {
   const int shapes[][2] = {{128, 256},  {4096, 4096}, {4096, 12288}, {200, 264},  {77, 8},
                            {1024, 1024}, {2048, 22016}, {8192, 4096}, {1152, 512}, {3000, 1000},
@@ -43,6 +65,16 @@ int main() {
     }
     checked += 2;
   }
+  for (int N : {8, 64, 96, 192, 264, 320, 352, 960, 1032, 1600, 1728, 4096})
+    for (int cols : {64, 32})
+      for (int ctas : {1, 2, 5}) {
+        int rc = check_staging<256>(3000, N, ctas, cols);
+        if (!rc) rc = check_staging<128>(3000, N, ctas, cols);
+        if (rc) {
+          std::fprintf(stderr, "staging: N=%d, %d columns a chunk: code %d\n", N, cols, rc);
+          return 1;
+        }
+      }
   // persistent attention: every item once, a CTA's items end at the first index past the end
   for (int ctas = 1; ctas <= 150; ctas += 7)
     for (int total = ctas; total <= 1100; total += 37) {
