@@ -69,6 +69,20 @@ def test_large_tensors_bit_exact(dtype, bits, block, tail):
     assert torch.equal(d.cpu().isnan(), dc.isnan())
 
 
+@pytest.mark.parametrize("bits", [1, 2, 4, 8])
+@pytest.mark.parametrize("n", [4097, (1 << 20) + 9])
+@pytest.mark.parametrize("before", [1, 2, 3, 4, 5, 6, 8, 10, 62, 64])
+def test_random_stream_index_wraps_inside_a_group(n, bits, before):
+    """The element index of the random stream is taken modulo 2^32 before it is halved: offsets
+    that put 2^32 inside a group of eight (2, 4 or 6 before it, alone or in a later group) and
+    between two groups, for the kernels of small and of large tensors."""
+    x = torch.randn(n, generator=torch.Generator().manual_seed(bits))
+    kw = dict(block_size=256, stochastic_rounding=True, sr_seed=13, sr_offset=2 ** 32 - before)
+    p, s, _ = Q.quantize_pack_tensor_blockwise(x.cuda(), bits, **kw)
+    pc, sc, _ = Q.quantize_pack_tensor_blockwise(x, bits, **kw)
+    assert torch.equal(s.cpu(), sc) and torch.equal(p.cpu(), pc)
+
+
 def test_blockwise_unaligned_view_and_zero_blocks():
     x = torch.randn(5003)
     x[256:512] = 0
