@@ -1140,7 +1140,7 @@ int bcom_rmsnorm_fwd(const void* x, const void* w, void* y, void* rstd, int rows
   cudaStream_t st = (cudaStream_t)stream;
   // a row is NV x 8 elements of up to 256 threads; few enough CTAs that each has a next row
   const int vecs = H / 8;
-  if (vecs > 8 * 256) {
+  if (vecs > 8 * 256 || vecs == 0) {
     rmsnorm_fwd_wide_kernel<<<rows < 148 * 8 ? rows : 148 * 8, 256, 0, st>>>(
         (const bf16*)x, (const bf16*)w, (bf16*)y, (float*)rstd, rows, H, eps);
     return (int)cudaGetLastError();
@@ -1244,6 +1244,7 @@ int bcom_layernorm_bwd(const void* dy, const void* x, const void* w, const void*
 // out[c] += sum over rows of x[row, c] (bf16 [rows, C], C % 8 == 0, 16-byte aligned; out fp32).
 // `partials`: fp32 scratch of bcom_colsum_strips(rows, C) * C elements.
 int bcom_colsum_strips(long long rows, int C) {
+  if (C <= 0) return 1;
   const int col_tiles = (C / 8 + 127) / 128;
   long long strips = (148LL * 8 + col_tiles - 1) / col_tiles;
   if (strips > (rows + 3) / 4) strips = (rows + 3) / 4;
@@ -1265,7 +1266,7 @@ int bcom_colsum_bf16(const void* x, void* out_fp32, void* partials, long long ro
 
 int bcom_bias_gelu_fwd(const void* x, const void* bias, void* y, long long rows, int C,
                        void* stream) {
-  if (rows <= 0) return 0;
+  if (rows <= 0 || C == 0) return 0;
   if (C % 8) return (int)cudaErrorInvalidValue;
   const int col_tiles = (C / 8 + 127) / 128;
   long long strips = (148LL * 16 + col_tiles - 1) / col_tiles;
@@ -1279,7 +1280,7 @@ int bcom_bias_gelu_fwd(const void* x, const void* bias, void* y, long long rows,
 // dbias: fp32 [C], accumulated into.
 int bcom_bias_gelu_bwd(const void* dy, const void* x, const void* bias, void* dx,
                        void* dbias_fp32, long long rows, int C, void* stream) {
-  if (rows <= 0) return 0;
+  if (rows <= 0 || C == 0) return 0;
   if (C % 8) return (int)cudaErrorInvalidValue;
   const int threads = 128;
   const int col_tiles = (C / 8 + threads - 1) / threads;
@@ -1301,6 +1302,7 @@ static int launch_rope(const void* src, void* dst, const void* cos_t, const void
     return (int)cudaErrorInvalidValue;
   const bool tables_aligned = (((uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0;
   const int items = heads * (head_dim / 16) + (out_of_place ? (width - heads * head_dim) / 8 : 0);
+  if (items <= 0) return 0;  // no heads
   const int cols = (items + 255) / 256;
   long long rows = (148LL * 16 + cols - 1) / cols;
   if (rows > tokens) rows = tokens;
