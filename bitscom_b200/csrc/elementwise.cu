@@ -705,10 +705,10 @@ rope_kernel(const bf16* src, bf16* dst, const float* __restrict__ cos_t,
 // Two independent 8-element groups per thread and iteration: all loads of both are issued
 // before the first result is needed (one group per iteration left the kernels at half the copy
 // rate: too few bytes in flight per thread for five streams).
-// silu(g) = g / (1 + e^-g): the approximate division (2 ulp in fp32; 0 beyond 2^126) keeps the
-// kernels at the memory's pace, the IEEE one made the forward kernel wait for its instructions
-// (4096 x 11008: 62 us, 47 us now).
-__device__ __forceinline__ float silu(float g) { return __fdividef(g, 1.0f + __expf(-g)); }
+// silu(g) = g / (1 + e^-g) with the IEEE division, as in the backward kernel.  The forward kernel
+// waits for it (4096 x 11008: 63 us against 51 with __fdividef), but __fdividef returns 0 for
+// a denominator above 2^126, which gates below -87 reach, and is 2 ulp off elsewhere.
+__device__ __forceinline__ float silu(float g) { return g / (1.0f + __expf(-g)); }
 
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ h, long long tokens, int F) {

@@ -160,6 +160,20 @@ def test_cross_entropy_loss_and_grad(rows, V):
     assert torch.allclose(work.grad.float(), ref_in.grad, rtol=5e-2, atol=2e-4)
 
 
+def test_swiglu_over_the_range_of_gates():
+    """Gates from -88.5 (1 + e^-g near the largest fp32) to 88, with ups that bring the products to
+    where bf16 has its full precision.  One rounding to bf16 (8 bits: 2^-8) and an exponential that is off by
+    2 + 1.2 |g| ulp of fp32 (2^-16)."""
+    g = torch.arange(-177, 177, device="cuda").double() / 2
+    silu = g / (1 + torch.exp(-g))
+    up = torch.exp2(-torch.floor(torch.log2(silu.abs().clamp_min(2.0 ** -122))))  # at most 2^122
+    gu = torch.cat([g, up]).to(torch.bfloat16).repeat(5, 1)
+    gu = torch.nn.functional.pad(gu.view(5, 2, -1), (0, 6)).reshape(5, -1).contiguous()
+    out = K.swiglu(gu)[:, :g.numel()].double()
+    want = silu * up
+    assert ((out - want).abs() <= (2.0 ** -8 + 2.0 ** -16) * want.abs()).all()
+
+
 @pytest.mark.parametrize("rows,V", [(3, 8184), (5, 8192), (700, 38272), (450, 38400), (300, 50432),
                                     (299, 57728), (7, 57856)])
 @pytest.mark.parametrize("upstream", [1.0, -2.5])
