@@ -199,6 +199,48 @@ def test_cross_entropy_vocabulary_rows(rows, V, upstream):
     assert torch.allclose(work.grad.float(), ref_in.grad, rtol=2 ** -7, atol=1e-9)
 
 
+@pytest.mark.parametrize("V", [512, 8192, 40960])
+def test_cross_entropy_small_probabilities(V):
+    """Probabilities down to e^-100 in the gradient, which a large loss scale makes visible: below
+    2^-126 they are subnormal in fp32 and must not be lost before the scaling.  An exponential of
+    |x| <= 126 is off by 2 + 1.2 |x| ulp (2^-16), subnormal results
+    have a spacing of 2^-149, bf16 rounds to 2^-8."""
+    z = torch.full((3, V), -120.0, device="cuda")
+    z[:, 8:209] = -torch.arange(201, device="cuda") / 2
+    z[:, 16:24] = float("-inf")
+    z[:, 0] = 6.0
+    targets = torch.zeros(3, dtype=torch.int64, device="cuda")
+    work = z.to(torch.bfloat16).requires_grad_()
+    assert torch.equal(work.detach().float(), z)
+    scale = 3 * 2.0 ** 100
+    K.cross_entropy(work * 1.0, targets, ignore_index=-100, loss_scale=scale).backward()
+    p = torch.softmax(z.double(), -1)
+    want = p * 2.0 ** 100
+    bound = want * (2.0 ** -8 + 2.0 ** -15) + 2.0 ** -149 * 2.0 ** 100
+    assert ((work.grad.double() - want).abs() <= bound)[:, 1:].all()
+
+
+def test_cross_entropy_sum_of_exponentials():
+    """loss = log(1 + (V - 1) e^x) for rows whose other words are all x below the target, against 64
+    bits: a term is off by (2 + 1.2 |x|) 2^-23, the whole sum by a rounding (2^-24 of it) at each of
+    16 additions that contain the target's 1 (4 of a thread, 2 + 5 of a warp, 4 of the warps), the
+    logarithm and the last additions by 2^-22 of the loss."""
+    V = 8192
+    x = -torch.arange(0, 97, device="cuda").double() / 4
+    z = x[:, None].repeat(1, V)
+    targets = torch.arange(x.numel(), device="cuda") * 80
+    z[torch.arange(x.numel(), device="cuda"), targets] = 0.0
+    logits = z.to(torch.bfloat16)
+    assert torch.equal(logits.double(), z)
+    for i in range(x.numel()):
+        loss = K.cross_entropy(logits[i:i + 1].clone(), targets[i:i + 1], ignore_index=-100).double()
+        rest = (V - 1) * torch.exp(x[i])
+        want = torch.log1p(rest)
+        bound = rest / (1 + rest) * (2 - 1.2 * x[i]) * 2.0 ** -23 + 16 * 2.0 ** -24
+        assert (loss - want).abs() <= bound + 2.0 ** -22 * want
+    K.check_status()
+
+
 def test_embedding_fwd_bwd():
     V, H, T = 1000, 256, 300
     table = _bf(V, H, seed=9).requires_grad_()
