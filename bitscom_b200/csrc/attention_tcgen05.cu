@@ -1416,9 +1416,11 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
           for (int v = 0; v < 8; ++v) {
             const float4 l = *reinterpret_cast<const float4*>(lse + v * 4);
             const float ls[4] = {l.x, l.y, l.z, l.w};
+            // exp2f keeps results below 2^-126, which a large dO can make count (with ex2_fast
+            // 269 instead of 271 us for the whole backward pass at B2 S2048 H32 D128)
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-              pt[v * 4 + u] = ex2_fast(__uint_as_float(r[v * 4 + u]) * p.scale_log2 - ls[u]);
+              pt[v * 4 + u] = exp2f(__uint_as_float(r[v * 4 + u]) * p.scale_log2 - ls[u]);
           }
         }
         if (i == 0) {  // the block on the diagonal: query >= key

@@ -1,5 +1,6 @@
 """tcgen05 causal attention (forward + backward) against fp32 SDPA on the same inputs."""
 
+import math
 import os
 
 import pytest
@@ -131,6 +132,35 @@ def test_persistent_kernels_match_reference(B, S, nh, growth, hd):
         got, want = x.grad[:, lo:lo + H].float(), xr.grad[:, lo:lo + H]
         e = (got - want).abs().max().item()
         assert e < 2 ** -6 * want.abs().max().item(), f"{name} max err {e}"
+
+
+@pytest.mark.parametrize("hd", [128, 64])
+@pytest.mark.parametrize("exponent", [-129, -140])
+def test_backward_of_small_probabilities(hd, exponent):
+    """One query that gives a key the probability 2^exponent, below fp32's normal range, and an
+    output gradient that makes it count: P must reach dS as it is (dQ, dK), and P^T dO as far as bf16
+    has it (dv of 2^-129: subnormal spacing 2^-133).  ex2 of an argument rounded to 2^-17 and one
+    rounding to bf16; 2^-140 has 9 bits in fp32."""
+    S, scale = 128, hd ** -0.5
+    qkv = torch.zeros(S, 3 * hd, device="cuda")
+    qkv[S - 1, 0] = 1.0
+    qkv[0, hd] = (exponent + 7) * math.log(2) / scale   # 127 other keys share the rest
+    qkv[0, 2 * hd + 1] = 2.0
+    x = qkv.to(torch.bfloat16).requires_grad_()
+    d_out = torch.zeros(S, hd, device="cuda", dtype=torch.bfloat16)
+    d_out[S - 1] = 2.0 ** 115
+    A.attention(x, 1, S, 1, hd).backward(d_out)
+    xr = x.detach().double().requires_grad_()
+    q, k, v = xr[:, :hd], xr[:, hd:2 * hd], xr[:, 2 * hd:]
+    causal = torch.ones(S, S, dtype=torch.bool, device="cuda").tril()
+    p = torch.softmax((q @ k.t() * scale).masked_fill(~causal, float("-inf")), -1)
+    (p @ v).backward(d_out.double())
+    assert 2.0 ** (exponent - 1) < p[S - 1, 0].item() < 2.0 ** (exponent + 1)
+    got, want = x.grad.double(), xr.grad
+    for row, col in ((S - 1, 0), (0, hd)):  # dq of the query, dk of the key
+        assert abs(got[row, col] - want[row, col]) <= 2.0 ** -6 * abs(want[row, col])
+    if exponent > -133:
+        assert abs(got[0, 2 * hd] - want[0, 2 * hd]) <= 2.0 ** -4 * abs(want[0, 2 * hd])
 
 
 def test_attention_second_call_reuses_zeroed_scratch():
