@@ -200,8 +200,9 @@ class RopeQKFunction(torch.autograd.Function):
         heads, head_dim, seq = ctx.meta
         d = dqkv.contiguous()
         if d.data_ptr() == dqkv.data_ptr():
-            if d.is_cuda and not torch.is_grad_enabled():
+            if d.is_cuda and not torch.is_grad_enabled() and d.data_ptr() % 16 == 0:
                 # the incoming gradient is not ours to change: rotate q and k, copy v, in one pass
+                # (a gradient that is not 16-byte aligned is cloned, which aligns it)
                 out = torch.empty_like(d)
                 rows = d.view(-1, d.shape[-1])
                 check(_need().bcom_rope_copy(

@@ -160,6 +160,21 @@ def test_cross_entropy_loss_and_grad(rows, V):
     assert torch.allclose(work.grad.float(), ref_in.grad, rtol=5e-2, atol=2e-4)
 
 
+@pytest.mark.parametrize("offset", [0, 1, 4, 8])
+def test_rope_backward_takes_any_alignment(offset):
+    """A contiguous gradient that starts anywhere in its storage: the same result, and the gradient
+    is left as it was."""
+    B, S, nh, hd = 2, 64, 2, 64
+    cos, sin = K.rope_tables(S, hd)
+    x = _bf(B * S, 3 * nh * hd, seed=31).requires_grad_()
+    grad = _bf(1, B * S * 3 * nh * hd + offset, seed=32)[0][offset:].view(B * S, -1)
+    assert grad.is_contiguous() and grad.data_ptr() % 16 == 2 * offset % 16
+    before = grad.clone()
+    aligned, got = (torch.autograd.grad(K.rope_qk_(x * 1.0, cos, sin, nh, hd, S), x, g)[0]
+                    for g in (before, grad))
+    assert torch.equal(got, aligned) and torch.equal(grad, before)
+
+
 def test_swiglu_over_the_range_of_gates():
     """Gates from -88.5 (1 + e^-g near the largest fp32) to 88, with ups that bring the products to
     where bf16 has its full precision.  One rounding to bf16 (8 bits: 2^-8) and an exponential that is off by
