@@ -37,7 +37,7 @@ LIBRARIES: Dict[str, dict] = {
     "bcom_cpu": {"sources": ["cpu_codec.cc"], "deps": [], "flags": [], "host_only": True},
     "bcom_llama": {"sources": ["gemm_tcgen05.cu", "attention_tcgen05.cu", "elementwise.cu"],
                    "deps": ["tc_common.cuh", "gemm_epilogue.cuh", "gemm_schedule.cuh",
-                            "attention_schedule.cuh", "no_alloc.h"],
+                            "attention_schedule.cuh", "rope_chunks.cuh", "no_alloc.h"],
                    "flags": []},
     # CTA-pair GEMM (opt-in variant): a library of its own, so that it can be left out of a
     # deployment without touching the default kernels

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "rope_chunks.cuh"
 #include "tc_common.cuh"
 
 namespace ew {
@@ -636,7 +637,7 @@ template <bool OUT_OF_PLACE>
 __global__ void __launch_bounds__(256)
 rope_kernel(const bf16* src, bf16* dst, const float* __restrict__ cos_t,
             const float* __restrict__ sin_t, int tokens, int heads, int head_dim,
-            long long row_stride, int width, int seq, float sign, bool tables_aligned) {
+            long long row_stride, int width, int seq, int pos0, float sign, bool tables_aligned) {
   const int half = head_dim / 2;
   const int vec_per_head = half / 8;
   const int rotated = heads * vec_per_head;
@@ -659,7 +660,7 @@ rope_kernel(const bf16* src, bf16* dst, const float* __restrict__ cos_t,
   const int h = j / vec_per_head, v = j - h * vec_per_head;
   const long long col = (long long)h * head_dim + v * 8;
   auto rotate = [&](int t, const uint4& qa, const uint4& qb) {
-    const int pos = t % seq;
+    const uint32_t pos = ((uint32_t)t + (uint32_t)pos0) % (uint32_t)seq;
     const float* c = cos_t + (size_t)pos * half + v * 8;
     const float* s = sin_t + (size_t)pos * half + v * 8;
     float cs[8], sn[8];
@@ -1299,26 +1300,27 @@ static int launch_rope(const void* src, void* dst, const void* cos_t, const void
                        int seq, int backward, bool out_of_place, void* stream) {
   if (tokens <= 0) return 0;
   // 16-byte accesses: halves of whole 8-element groups, rows and bases aligned
-  if (head_dim % 16 || row_stride % 8 || width % 8 || tokens > 0x7fffffff ||
+  if (seq <= 0 || head_dim % 16 || row_stride % 8 || width % 8 ||
       (((uintptr_t)src | (uintptr_t)dst) & 15))
     return (int)cudaErrorInvalidValue;
   const bool tables_aligned = (((uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0;
   const int items = heads * (head_dim / 16) + (out_of_place ? (width - heads * head_dim) / 8 : 0);
   if (items <= 0) return 0;  // no heads
   const int cols = (items + 255) / 256;
-  long long rows = (148LL * 16 + cols - 1) / cols;
-  if (rows > tokens) rows = tokens;
-  if (rows > 65535) rows = 65535;
-  const dim3 grid(cols, (unsigned)rows);
-  if (out_of_place)
-    rope_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(
-        (const bf16*)src, (bf16*)dst, (const float*)cos_t, (const float*)sin_t, (int)tokens, heads,
-        head_dim, row_stride, width, seq, backward ? -1.0f : 1.0f, tables_aligned);
-  else
-    rope_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(
-        (const bf16*)src, (bf16*)dst, (const float*)cos_t, (const float*)sin_t, (int)tokens, heads,
-        head_dim, row_stride, width, seq, backward ? -1.0f : 1.0f, tables_aligned);
-  return (int)cudaGetLastError();
+  const long long most_rows = (148LL * 16 + cols - 1) / cols;
+  auto kernel = out_of_place ? rope_kernel<true> : rope_kernel<false>;
+  for (long long first = 0; first < tokens;) {
+    const RopeChunk part = rope_chunk(tokens, seq, first);
+    const long long rows = most_rows < part.tokens ? most_rows : part.tokens;
+    kernel<<<dim3(cols, (unsigned)rows), 256, 0, (cudaStream_t)stream>>>(
+        (const bf16*)src + first * row_stride, (bf16*)dst + first * row_stride,
+        (const float*)cos_t, (const float*)sin_t, part.tokens, heads, head_dim, row_stride, width,
+        seq, part.position, backward ? -1.0f : 1.0f, tables_aligned);
+    const cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) return (int)err;
+    first += part.tokens;
+  }
+  return 0;
 }
 
 // In place on the first heads * head_dim columns of rows `row_stride` apart.

@@ -9,6 +9,7 @@
 #define __device__
 #include "attention_schedule.cuh"
 #include "gemm_schedule.cuh"
+#include "rope_chunks.cuh"
 
 template <int BM, int BN>
 static int check(int M, int N) {
@@ -84,6 +85,21 @@ int main() {
           ++taken[attn_sched::item_index(c, ctas, j)];
       for (int t : taken)
         if (t != 1) return 9;
+    }
+  // RoPE launches: every token once and in order at its own position, and a thread that steps past
+  // the last token by two rows of the largest grid stays within 32 bits
+  for (long long tokens : {1LL, 4096LL, 1LL << 30, (1LL << 30) + 1, (1LL << 31) - 1, (1LL << 31) + 5,
+                           7000000001LL})
+    for (int seq : {1, 127, 2048, 1 << 30, 2147483647}) {
+      long long first = 0;
+      while (first < tokens) {
+        const ew::RopeChunk part = ew::rope_chunk(tokens, seq, first);
+        if (part.first != first || part.tokens < 1 || part.position != first % seq) return 11;
+        if ((long long)part.tokens + 4 * 65535 > 2147483647LL) return 12;
+        if ((long long)part.tokens + part.position > 4294967295LL) return 13;
+        first += part.tokens;
+      }
+      if (first != tokens) return 14;
     }
   // shares of K: in order, without gaps, none empty
   for (int kb = 1; kb <= 200; ++kb)

@@ -18,6 +18,7 @@ CALLS = {
     "bias_gelu_bwd": ("lib.bcom_bias_gelu_bwd(z, z, z, z, z, ll(5), 0, z)", 0),
     "rope": ("lib.bcom_rope(z, z, z, ll(5), 0, 64, ll(64), 128, 0, z)", 0),
     "rope_head_dim": ("lib.bcom_rope(z, z, z, ll(5), 4, 0, ll(64), 128, 0, z)", 0),
+    "rope_no_positions": ("lib.bcom_rope(z, z, z, ll(5), 4, 64, ll(256), 0, 0, z)", 1),
     "rope_copy": ("lib.bcom_rope_copy(z, z, z, z, ll(5), 0, 64, ll(64), 0, 128, 1, z)", 0),
 }
 
