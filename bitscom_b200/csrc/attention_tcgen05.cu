@@ -1697,10 +1697,13 @@ attention_bwd_pipelined_kernel(const __grid_constant__ CUtensorMap tm_qkv,  // b
 // delta[b, h, s] = sum_d dO * O.  HD / 8 adjacent lanes share a (token, head) and load 16 bytes
 // each of both tensors; two of them per thread are in flight.  (One warp per pair with 4 or 8
 // bytes per lane: 25 us for 67 MB at B2 S2048 H32 D128, 24 us for 34 MB at B8 S1024 H16 D64.)
+// They also clear their 8 columns of the dQ accumulator, so that the scratch a call is given may
+// hold anything and is never shared with another call.
 template <int HD>
 __global__ void __launch_bounds__(256)
 attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                       float* __restrict__ delta, int batch, int seq, int heads, bool aligned) {
+                       float* __restrict__ delta, float* __restrict__ dq_acc, int batch, int seq,
+                       int heads, bool aligned) {
   constexpr int LANES = HD / 8;
   const long long total = (long long)batch * seq * heads;  // (token, head) pairs, head fastest
   const int sub = threadIdx.x % LANES;
@@ -1733,6 +1736,10 @@ attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16*
       delta[((size_t)b * heads + h) * seq + sp] = s;
     }
   };
+  auto clear = [&](long long pair) {
+    float4* dst = reinterpret_cast<float4*>(dq_acc + pair * HD + sub * 8);
+    dst[0] = dst[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  };
   // the loop bound is uniform over a warp: its lanes' pairs are adjacent, the shuffles need all
   for (long long p0 = first; p0 - threadIdx.x / LANES < total; p0 += 2 * stride) {
     const long long p1 = p0 + stride;
@@ -1740,22 +1747,24 @@ attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16*
     if (p0 < total) {
       a0 = load(o + p0 * HD + sub * 8);
       g0 = load(d_o + p0 * HD + sub * 8);
+      clear(p0);
     }
     if (p1 < total) {
       a1 = load(o + p1 * HD + sub * 8);
       g1 = load(d_o + p1 * HD + sub * 8);
+      clear(p1);
     }
     finish(dot(a0, g0), p0);
     finish(dot(a1, g1), p1);
   }
 }
 
-// dqkv[:, 0:H] = bf16(dq_acc); dq_acc is left zeroed for the next call.  A thread owns one
+// dqkv[:, 0:H] = bf16(dq_acc).  A thread owns one
 // float4 column (blockIdx.x, threadIdx.x) and walks the tokens four at a time with all four
 // loads issued before the first store: one load in flight per thread, and a 64-bit division per
 // element to find its row, made this pass take as long as a quarter of the backward kernel.
 __global__ void __launch_bounds__(256)
-attention_dq_finish_kernel(float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv,
+attention_dq_finish_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv,
                            long long tokens, int H) {
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= H / 4) return;
@@ -1769,7 +1778,6 @@ attention_dq_finish_kernel(float* __restrict__ dq_acc, __nv_bfloat16* __restrict
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (t0 + u < tokens) {
-        *reinterpret_cast<float4*>(dq_acc + (t0 + u) * H + c) = make_float4(0.f, 0.f, 0.f, 0.f);
         uint2 o;
         o.x = pack_bf16(v[u].x, v[u].y);
         o.y = pack_bf16(v[u].z, v[u].w);
@@ -1915,10 +1923,9 @@ static int launch_bwd(const void* qkv, const void* out, const void* d_out, const
   const bool pipelined =
       g_bwd_dq_variant == 2 && !((uintptr_t)lse2 & 15) && !((uintptr_t)delta & 15);
   const bool tma_dq = g_bwd_dq_variant >= 1;
+  if ((uintptr_t)dq_acc & 15) return 1007;
   if (tma_dq) {
-    if (((uintptr_t)dq_acc & 15) ||
-        make_map_f32(&tm_dq, dq_acc, tokens, H, 32, pipelined ? 32 : 128))
-      return 1007;
+    if (make_map_f32(&tm_dq, dq_acc, tokens, H, 32, pipelined ? 32 : 128)) return 1007;
   } else {
     tm_dq = tm_do;  // unused by the kernel
   }
@@ -1927,8 +1934,8 @@ static int launch_bwd(const void* qkv, const void* out, const void* d_out, const
     const long long want = (tokens * heads + per_cta - 1) / per_cta;
     const int grid = (int)(want < 148 * 8 ? want : 148 * 8);
     attention_delta_kernel<HD><<<grid, 256, 0, st>>>((const __nv_bfloat16*)out,
-                                                     (const __nv_bfloat16*)d_out, delta, batch,
-                                                     seq, heads,
+                                                     (const __nv_bfloat16*)d_out, delta, dq_acc,
+                                                     batch, seq, heads,
                                                      (((uintptr_t)out | (uintptr_t)d_out) & 15) == 0);
   }
   BwdParams p;
@@ -2020,8 +2027,8 @@ int bcom_attention_set_fwd_variant(int variant) {
 }
 
 // d_out: [batch*seq, heads*head_dim]; dqkv (written): [batch*seq, 3*heads*head_dim];
-// dq_acc: fp32 [batch*seq, heads*head_dim] scratch, must be zero on entry and is zero on exit;
-// delta: fp32 [batch, heads, seq] scratch.
+// dq_acc: fp32 [batch*seq, heads*head_dim] scratch, 16-byte aligned; delta: fp32 [batch, heads, seq]
+// scratch.  Both may hold anything and belong to the call until it has run.
 int bcom_attention_bwd(const void* qkv, const void* out, const void* d_out, const void* lse2,
                        void* dqkv, void* dq_acc, void* delta, int batch, int seq, int heads,
                        int head_dim, float scale, void* stream) {
@@ -2112,9 +2119,6 @@ int bcom_attention_bwd_no_alloc(const void* qkv, const void* out, const void* d_
   cudaStream_t st = (cudaStream_t)stream;
   float* dq_acc = reinterpret_cast<float*>(scratch);
   float* delta = reinterpret_cast<float*>(scratch + dq_bytes);
-  // the accumulator must start at zero; the array still holds the previous call's data
-  err = cudaMemsetAsync(dq_acc, 0, dq_bytes, st);
-  if (err != cudaSuccess) return (int)err;
   return launch_bwd<128>(qkv, out, d_out, lse2, dqkv, dq_acc, delta, batch, seq, heads, scale,
                          st);
 }

@@ -40,7 +40,7 @@ extern "C" {
 //     other value is the cudaError_t of the failing runtime call (for example 2,
 //     cudaErrorMemoryAllocation, from the module load described above).
 //   * All calls on a device share the one array, and it keeps whatever the previous call
-//     left: the accumulator part is cleared on the stream at the start of every call.
+//     left: the accumulator part is cleared on the stream by every call's first kernel.
 //     Two calls whose kernels overlap on the GPU (different streams, no ordering) race
 //     on the array and corrupt each other's gradients: order them.
 //

@@ -7,7 +7,6 @@ from __future__ import annotations
 import ctypes
 import math
 import os
-from typing import Dict, Tuple
 
 import torch
 
@@ -15,7 +14,6 @@ from . import _native
 from ._native import NativeError, check, ptr, stream_ptr
 
 _lib = None
-_scratch: Dict[Tuple, torch.Tensor] = {}
 # forward kernels: "simple" alternates MMA and softmax inside a CTA; "pipelined" has an issuer
 # warp, double-buffered scores in TMEM and the output accumulated in TMEM; "dual" (default) has
 # two query tiles per persistent CTA whose products and softmax overlap
@@ -88,13 +86,6 @@ def check_status(clear: bool = True) -> None:
         raise NativeError(f"attention kernel timed out at wait {out[0]} (cta {out[1]})")
 
 
-def _zero_scratch(key, shape, device) -> torch.Tensor:
-    buf = _scratch.get(key)
-    if buf is None:
-        buf = _scratch[key] = torch.zeros(shape, dtype=torch.float32, device=device)
-    return buf
-
-
 class AttentionFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, batch, seq, heads, head_dim):
@@ -123,7 +114,8 @@ class AttentionFunction(torch.autograd.Function):
         d_out = d_out.contiguous()
         dqkv = torch.empty_like(q2)
         dev = q2.device
-        dq_acc = _zero_scratch(("dq", batch * seq, H, dev.index), (batch * seq, H), dev)
+        # private to the call: passes on other streams or threads have accumulators of their own
+        dq_acc = torch.empty(batch * seq, H, dtype=torch.float32, device=dev)
         delta = torch.empty(batch, heads, seq, dtype=torch.float32, device=dev)
         check(lib.bcom_attention_bwd(ptr(q2), ptr(out), ptr(d_out), ptr(lse), ptr(dqkv),
                                      ptr(dq_acc), ptr(delta), batch, seq, heads, head_dim,

@@ -9,7 +9,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 if torch.cuda.is_available():
-    from bitscom_b200.ops import attention as A
+    from bitscom_b200.ops import _native, attention as A
 
 
 def _ref(qkv, B, S, nh, hd):
@@ -174,6 +174,65 @@ def test_attention_second_call_reuses_zeroed_scratch():
         A.attention(x, B, S, nh, hd).backward(d_out)
         grads.append(x.grad.clone())
     assert torch.equal(grads[0], grads[1])
+
+
+@pytest.mark.parametrize("variant", ["atomic", "tma", "pipelined"])
+@pytest.mark.parametrize("B,S,nh,hd", [(1, 128, 1, 128), (3, 256, 5, 64), (1, 384, 3, 128)])
+def test_backward_scratch_may_hold_anything(variant, B, S, nh, hd):
+    """The dQ accumulator and the row sums are given to the C entry full of other values."""
+    lib, stream, H, scale = A._get(), _native.stream_ptr(), nh * hd, hd ** -0.5
+    qkv = (torch.randn(B * S, 3 * H, device="cuda") * 0.5).to(torch.bfloat16)
+    d_out = (torch.randn(B * S, H, device="cuda") * 0.5).to(torch.bfloat16)
+    out, lse = torch.empty_like(d_out), torch.empty(B, nh, S, device="cuda")
+    check = _native.check
+    check(lib.bcom_attention_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S, nh, hd, scale,
+                                 stream), "fwd")
+    got = []
+    before = A.set_backward_dq_variant(variant)
+    try:
+        for fill in (0.0, 3.0, float("nan")):
+            acc = torch.full((B * S, H), fill, device="cuda")
+            delta = torch.full((B, nh, S), fill, device="cuda")
+            got.append(torch.empty_like(qkv))
+            check(lib.bcom_attention_bwd(
+                qkv.data_ptr(), out.data_ptr(), d_out.data_ptr(), lse.data_ptr(), got[-1].data_ptr(),
+                acc.data_ptr(), delta.data_ptr(), B, S, nh, hd, scale, stream), "bwd")
+    finally:
+        A.set_backward_dq_variant(before)
+    torch.cuda.synchronize()
+    A.check_status()
+    for other in got[1:]:  # dq is a sum in any order: up to 3 terms here
+        assert torch.equal(other[:, H:], got[0][:, H:])
+        assert torch.allclose(other[:, :H].float(), got[0][:, :H].float(), rtol=2 ** -7, atol=1e-5)
+
+
+def test_backward_passes_on_two_streams_at_once():
+    """Passes of one shape on two streams, queued behind a wait so that they run together.  Two key
+    blocks per sequence: a sum of two dQ terms does not depend on their order."""
+    B, S, nh, hd = 24, 256, 8, 128
+    H, work = nh * hd, []
+    for seed in range(2):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        qkv = (torch.randn(B * S, 3 * H, device="cuda", generator=g) * 0.5).to(torch.bfloat16)
+        d_out = (torch.randn(B * S, H, device="cuda", generator=g) * 0.5).to(torch.bfloat16)
+        qkv.requires_grad_()
+        out = A.attention(qkv, B, S, nh, hd)
+        want = torch.autograd.grad(out, qkv, d_out, retain_graph=True)[0]
+        work.append((qkv, d_out, out, want, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    grads = [[], []]
+    for qkv, d_out, _, _, stream in work:
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(20_000_000)
+    for _ in range(8):
+        for i, (qkv, d_out, _, _, stream) in enumerate(work):
+            with torch.cuda.stream(stream):
+                out = A.attention(qkv, B, S, nh, hd)
+                grads[i].append(torch.autograd.grad(out, qkv, d_out)[0])
+    torch.cuda.synchronize()
+    A.check_status()
+    for got, (_, _, _, want, _) in zip(grads, work):
+        assert all(torch.equal(g, want) for g in got)
 
 
 @pytest.mark.performance
