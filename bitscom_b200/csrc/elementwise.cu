@@ -847,7 +847,7 @@ cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ ta
 // three persistent CTAs per SM work on rows of their own, so that one waits for its copy or for
 // its reduction while the others compute: with the special-function unit busy for half of the
 // time that the row's bytes take, one row at a time per SM (with the next one prefetched) came
-// to 111 / 356 us.  Measured: 108 / 340 us (4.9 TB/s, 0.74 of copy).
+// to 111 / 356 us.  Measured: 113 / 346 us (4.7 / 4.8 TB/s, 0.71 / 0.73 of copy).
 constexpr int kCeThreads = 512;
 constexpr unsigned long long kCeBudgetNs = 2000000000ull;
 
@@ -856,6 +856,7 @@ __device__ unsigned int g_ce_status;      // 1: a row's copy did not arrive with
 struct alignas(128) CeShared {
   float2 part[2][kCeThreads / 32];
   uint64_t full;
+  volatile int expired;  // 1 + the number of the CTA's row whose copy did not arrive
 };
 
 // (maximum, sum of e^(x - maximum)) of two sets; an empty or fully masked one is (-inf, 0)
@@ -881,6 +882,7 @@ cross_entropy_rows_kernel(bf16* __restrict__ logits, const long long* __restrict
   };
   if (tid == 0) {
     tc::mbar_init(&sh->full, 1);
+    sh->expired = 0;
     tc::fence_mbar_init();
     if (blockIdx.x < rows) load(blockIdx.x);
   }
@@ -889,17 +891,15 @@ cross_entropy_rows_kernel(bf16* __restrict__ logits, const long long* __restrict
   const int vec = V / 8;
   const float gscale = grad_scale[0];
   int it = 0;
-  unsigned long long budget = kCeBudgetNs;
   long long tgt = blockIdx.x < rows ? targets[blockIdx.x] : 0;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x, ++it) {
     // the next row's target is requested a row ahead: its latency would stall every row
     const long long next_tgt = row + gridDim.x < rows ? targets[row + gridDim.x] : 0;
     const bool ignored = tgt == ignore_index || tgt < 0 || tgt >= V;
-    if (!tc::mbar_wait(&sh->full, (uint32_t)it & 1u, budget)) {
-      // go on with what is there (a thread that left would leave the others in a barrier), but
-      // do not wait again
+    if (!tc::mbar_wait(&sh->full, (uint32_t)it & 1u, kCeBudgetNs)) {
+      // finish the row with what is there: a thread that left would leave the others in a barrier
       atomicCAS(&g_ce_status, 0u, 1u);
-      budget = 0;
+      sh->expired = it + 1;
     }
     float m = -INFINITY;
 #pragma unroll 4
@@ -954,6 +954,10 @@ cross_entropy_rows_kernel(bf16* __restrict__ logits, const long long* __restrict
     }
     tgt = next_tgt;
     __syncthreads();  // everybody has read the row
+    if (sh->expired == it + 1) {  // no further copy; the one under way gets another chance to land
+      if (tid == 0) (void)tc::mbar_wait(&sh->full, (uint32_t)it & 1u, kCeBudgetNs);
+      break;
+    }
     if (tid == 0 && row + gridDim.x < rows) load(row + gridDim.x);
   }
 }
