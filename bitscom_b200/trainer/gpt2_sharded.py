@@ -21,6 +21,7 @@ import time
 import torch
 import torch.distributed as dist
 
+from .. import ops
 from ..api import LowBitGroup
 from ..models.gpt2 import GPT2, GPT2Config
 from ..ops import nn as K
@@ -188,6 +189,7 @@ def main(argv=None):
         elapsed_ms = s.elapsed_time(e)
     else:
         elapsed_ms = (time.perf_counter() - t0) * 1e3
+    ops.check_status(dev)  # before anything is reported or saved
     ms = torch.tensor([elapsed_ms / args.steps], device=dev)
     if world > 1:
         dist.all_reduce(ms, op=dist.ReduceOp.MAX)

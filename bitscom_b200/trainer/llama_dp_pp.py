@@ -30,6 +30,7 @@ from typing import List, Optional, Tuple
 import torch
 import torch.distributed as dist
 
+from .. import ops
 from ..api import LowBitGroup
 from ..models.llama import LlamaConfig, LlamaStage
 from ..ops import nn as K
@@ -333,18 +334,8 @@ class LlamaTrainer:
         waits since the last check (it then returned early and its output is not valid).
         Synchronises the device, so call it where the step is synchronised anyway, and before
         a checkpoint replaces the last good file."""
-        from ..ops import attention as A
-        from ..ops import gemm as G
-        from ..ops import nn as K
-
-        if self.device.type != "cuda":
-            return
-        if G.available():
-            G.check_status()
-            K.check_status()
-        if A.available():
-            A.check_status()
-        if self.syncs:
+        ops.check_status(self.device)
+        if self.device.type == "cuda" and self.syncs:
             torch.cuda.synchronize(self.device)
             for sync in self.syncs:
                 sync.check(wait=True)

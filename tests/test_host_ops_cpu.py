@@ -7,6 +7,7 @@ import os
 import subprocess
 import sys
 
+import pytest
 import torch
 import torch.nn.functional as F
 
@@ -150,6 +151,27 @@ def test_gpt2_sharded_trainer_on_two_cpu_ranks(tmp_path):
         assert row["device"] == "cpu" and row["world"] == 2 and not row["fused_ops"]
         assert row["loss_last"] < row["loss_first"]
     assert abs(low["loss_last"] - dense["loss_last"]) < 0.05
+
+
+def test_trainers_ask_for_the_kernels_status(tmp_path, monkeypatch):
+    """A kernel that gave up on a wait ends a run before it reports or saves anything."""
+    from bitscom_b200 import ops
+    from bitscom_b200.trainer import gpt2_sharded, llama_dp_pp
+
+    def expired(device):
+        raise RuntimeError(f"a wait ran out on {device}")
+
+    monkeypatch.setattr(ops, "check_status", expired)
+    out = tmp_path / "rows.jsonl"
+    with pytest.raises(RuntimeError, match="a wait ran out"):
+        gpt2_sharded.main(["--device", "cpu", "--model", "tiny", "--steps", "1", "--warmup", "0",
+                           "--micro-batch", "1", "--out", str(out), "--output_dir",
+                           str(tmp_path / "ckpt")])
+    assert not out.exists() and not (tmp_path / "ckpt").exists()
+    trainer = object.__new__(llama_dp_pp.LlamaTrainer)
+    trainer.device, trainer.sync = torch.device("cpu"), None
+    with pytest.raises(RuntimeError, match="a wait ran out"):
+        trainer.check_kernels()
 
 
 def _gpt2(nproc, tmp_path, *extra):
