@@ -220,6 +220,32 @@ def test_linear_bias_gradient(rows, n, main):
 
 
 @pytest.mark.parametrize("plan", [-1, 0, 1, 3])
+@pytest.mark.parametrize("a_mn", [False, True])
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("M,N,K", [(128, 256, 256), (200, 264, 456), (8, 8, 200), (1032, 1000, 1024)])
+def test_each_kernel_in_every_form(monkeypatch, plan, a_mn, b_mn, M, N, K):
+    """The rule that picks a kernel sends shapes this small to the 128x128 form, so each kernel is
+    asked for by its plan: operand layouts, rows with a stride, bf16 and fp32 outputs inside a wider
+    matrix, overwriting and accumulating; exact on small integers."""
+    if plan < 0 and not G.pair_available():
+        pytest.skip("the CTA-pair library is not part of this installation")
+    monkeypatch.setattr(G, "_plan", lambda *a: plan)
+    ai, bi = (torch.randint(-3, 4, (rows + 8, cols + 24), device="cuda").to(torch.bfloat16)[8:, 8:-16]
+              for rows, cols in ((K, M) if a_mn else (M, K), (K, N) if b_mn else (N, K)))
+    ref = _ref(ai, bi, a_mn, b_mn)
+    kw = dict(a_mn_major=a_mn, b_mn_major=b_mn)
+    for dtype in (torch.bfloat16, torch.float32):
+        wide = torch.full((M, N + 16), 7.0, device="cuda", dtype=dtype)
+        out = G.gemm(ai, bi, out=wide[:, 8:8 + N], **kw)
+        assert torch.equal(out, ref.to(dtype))
+        want = (out.float() + ref).to(dtype)
+        G.gemm(ai, bi, out=out, accumulate=True, **kw)
+        assert torch.equal(out, want)
+        assert (wide[:, :8] == 7).all() and (wide[:, 8 + N:] == 7).all()
+    G.check_status()
+
+
+@pytest.mark.parametrize("plan", [-1, 0, 1, 3])
 @pytest.mark.parametrize("mn", [False, True])
 @pytest.mark.parametrize("N,K", [(64, 64), (96, 328), (192, 64), (320, 328), (352, 200), (1728, 128)])
 def test_several_tiles_per_cta_with_ragged_columns(monkeypatch, plan, mn, N, K):
