@@ -39,8 +39,8 @@ LIBRARIES: Dict[str, dict] = {
                    "deps": ["tc_common.cuh", "gemm_epilogue.cuh", "gemm_schedule.cuh",
                             "attention_schedule.cuh", "rope_chunks.cuh", "no_alloc.h"],
                    "flags": []},
-    # CTA-pair GEMM (opt-in variant): a library of its own, so that it can be left out of a
-    # deployment without touching the default kernels
+    # CTA-pair GEMM, the default for large products: a library of its own, so that it can be left
+    # out of a deployment, whose products then all take the one-CTA kernel
     "bcom_gemm2": {"sources": ["gemm_tcgen05_2cta.cu"],
                    "deps": ["tc_common.cuh", "gemm_epilogue.cuh", "gemm_schedule.cuh"],
                    "flags": []},

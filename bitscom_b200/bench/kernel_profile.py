@@ -241,7 +241,7 @@ def elementwise(args):
     for _ in range(args.warmup):
         K.cross_entropy(logits, tgt, 0)
     ms = _timed(lambda i: K.cross_entropy(logits, tgt, 0), args.iters)
-    rows.append(("cross_entropy_fwd_bwd", ms, 4 * T * V * 2))
+    rows.append(("cross_entropy_fwd_bwd", ms, 2 * T * V * 2))  # a row is read and written once
     n = 1 << 28
     master, grad = torch.randn(n, device="cuda"), torch.randn(n, device="cuda")
     opt = K.FlatAdamW(master, grad, torch.empty(n, device="cuda", dtype=torch.bfloat16))
@@ -348,9 +348,8 @@ def main(argv=None):
     ap.add_argument("--seq", type=int, default=2048)
     ap.add_argument("--heads", type=int, default=32)
     ap.add_argument("--head-dim", type=int, default=128, choices=[64, 128])
-    ap.add_argument("--fwd-variant", default="pipelined",
-                    choices=["simple", "pipelined"])
-    ap.add_argument("--bwd-dq", default="tma", choices=["atomic", "tma"])
+    ap.add_argument("--fwd-variant", default="dual", choices=["simple", "pipelined", "dual"])
+    ap.add_argument("--bwd-dq", default="pipelined", choices=["atomic", "tma", "pipelined"])
     ap.add_argument("--tokens", type=int, default=8192)
     ap.add_argument("--elems", type=int, default=1 << 25)
     ap.add_argument("--bits", type=int, default=4)

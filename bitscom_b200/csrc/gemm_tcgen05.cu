@@ -1,15 +1,18 @@
 // bf16 GEMM on the 5th-generation tensor cores (sm_100a): C[M,N] (+)= A x B with fp32
 // accumulation in tensor memory.
 //
-//   * persistent grid, one CTA per SM, static round-robin over 128x256 output tiles
-//     (grouped along M so that concurrently running CTAs share B tiles in L2);
+//   * persistent grid, one CTA per SM, static round-robin over work items: output tiles of
+//     128x256 or 128x128 (grouped along M so that concurrently running CTAs share B tiles in
+//     L2), the latter also with K shared out among several items per tile, whose fp32 partial
+//     tiles a second kernel adds up;
 //   * warp 0: TMA producer (cp.async.bulk.tensor 2-D tiles, 128-byte swizzle) into a
-//     4-stage shared-memory ring (48 KiB per stage);
-//   * warp 1: allocates 512 TMEM columns and issues tcgen05.mma (cta_group::1,
-//     M=128, N=256, K=16 per instruction) from one elected thread; tcgen05.commit
-//     releases ring stages and publishes finished accumulators;
-//   * warps 2-5: epilogue. Two 256-column accumulators alternate, so the epilogue of
-//     tile i (tcgen05.ld -> registers -> global) overlaps the main loop of tile i+1.
+//     192 KiB shared-memory ring (4 stages of 48 KiB or 6 of 32 KiB);
+//   * warp 1: allocates two accumulators of TMEM and issues tcgen05.mma (cta_group::1, M=128,
+//     N=256 or 128, K=16 per instruction): the whole warp walks the loop, an elected lane
+//     issues; tcgen05.commit releases ring stages and publishes finished accumulators;
+//   * warps 2-5: epilogue (gemm_epilogue.cuh). The two accumulators alternate, so the epilogue
+//     of item i (tcgen05.ld -> registers -> shared memory -> bulk tensor store or reduction)
+//     overlaps the main loop of item i+1.
 //
 // Operand layouts.  Either operand may be K-major (reduction dimension contiguous) or
 // MN-major (the other dimension contiguous); this covers forward (x W^T), data
@@ -429,6 +432,7 @@ int bcom_gemm_bf16_bias(const void* A, const void* B, void* C, const void* resid
                      (cudaStream_t)stream);
 }
 
+// The forms without a bias, and without a residual either, for C callers.
 int bcom_gemm_bf16_ex(const void* A, const void* B, void* C, const void* residual, int M, int N,
                       int K, long long lda, long long ldb, long long ldc, long long ldr,
                       int a_mn_major, int b_mn_major, int out_fp32, int accumulate, int max_ctas,

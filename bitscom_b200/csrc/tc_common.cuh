@@ -112,7 +112,7 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       : "r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
       : "memory");
 }
-// untiled bulk copies (both addresses 16-byte aligned, size a multiple of 16)
+// untiled bulk copy, global -> shared (both addresses 16-byte aligned, size a multiple of 16)
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes,
                                           uint64_t* bar) {
   asm volatile(
@@ -120,12 +120,6 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint3
       :
       : "r"(smem_u32(smem_dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
-}
-__device__ __forceinline__ void bulk_store(void* dst, const void* smem_src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-               :
-               : "l"(dst), "r"(smem_u32(smem_src)), "r"(bytes)
-               : "memory");
 }
 // 2-D tiled reduction, shared -> global: global[tile] += shared[tile], element-wise, in the
 // tensor map's data type.  Completion is tracked by bulk groups of the issuing thread.  The

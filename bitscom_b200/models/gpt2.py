@@ -139,8 +139,8 @@ class GPT2(torch.nn.Module):
         return hook
 
     def collect_autograd_grads(self, prefix: Optional[str] = None) -> None:
-        """Parameters updated by torch ops (LayerNorm, biases, position embedding) receive
-        ``.grad``; fold them into the flat fp32 gradient buffer.  ``prefix`` limits the pass
+        """Parameters whose gradients come from torch ops (the position embedding; LayerNorm and
+        the activation's bias without the fused ops) receive ``.grad``; fold them into the flat fp32 gradient buffer.  ``prefix`` limits the pass
         to the parameters whose name starts with it (one layer: ``"h3."``)."""
         want = None if prefix is None else prefix.replace(".", "_")
         for name, p in self.p.items():

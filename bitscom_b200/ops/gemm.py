@@ -28,10 +28,6 @@ def _get():
         lib = _native.load("bcom_llama")
         if lib is not None:
             vp, ll, ci = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
-            lib.bcom_gemm_bf16.argtypes = [vp, vp, vp, ci, ci, ci, ll, ll, ll, ci, ci, ci, ci,
-                                           ci, vp]
-            lib.bcom_gemm_bf16_ex.argtypes = [vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci, ci,
-                                              ci, ci, ci, vp]
             lib.bcom_gemm_bf16_bias.argtypes = [vp, vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci,
                                                 ci, ci, ci, ci, vp]
             lib.bcom_colsum_bf16.argtypes = [vp, vp, vp, ll, ci, vp]
@@ -56,10 +52,6 @@ def _get2():
             lib = None
         if lib is not None:
             vp, ll, ci = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
-            lib.bcom_gemm2_bf16.argtypes = [vp, vp, vp, ci, ci, ci, ll, ll, ll, ci, ci, ci, ci,
-                                            ci, vp]
-            lib.bcom_gemm2_bf16_ex.argtypes = [vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci,
-                                               ci, ci, ci, ci, vp]
             lib.bcom_gemm2_bf16_bias.argtypes = [vp, vp, vp, vp, vp, ci, ci, ci, ll, ll, ll, ll, ci,
                                                  ci, ci, ci, ci, vp]
             lib.bcom_gemm2_status.argtypes = [ctypes.POINTER(ctypes.c_uint * 4), ci]
