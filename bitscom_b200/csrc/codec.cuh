@@ -376,8 +376,8 @@ __device__ __forceinline__ Packed8<BITS> quant8_pack_lean(const float (&x)[GROUP
   const float y = __frcp_rn(sf);
   float f[GROUP];  // 2^23 + the element's 16 random bits
   if constexpr (SR) {
-    // the usual case: two elements share one hash, and the index does not pass 2^32 inside the group
-    // (there the pair number starts over, which a constant distance to the first pair's would miss)
+    // the usual case: two elements share one hash, and the index does not pass 2^32 inside the
+    // group (there the pair number starts over, which a constant distance would miss)
     if ((idx0 & 1u) == 0u && idx0 <= 0u - (uint32_t)GROUP) {
 #pragma unroll
       for (int i = 0; i < GROUP; i += 2) {

@@ -7,8 +7,8 @@
 //     B tile (that is, columns of C) in its own shared memory: 32 KiB per pipeline stage
 //     against 48 KiB for the same work per SM in the one-CTA kernel, so the ring is 6 stages
 //     deep and every B element is read from L2 once per pair instead of once per CTA;
-//   * one warp of the even CTA (the leader; its elected lane) issues tcgen05.mma.cta_group::2 with M = 256,
-//     N = 256, K = 16: the tensor cores of both SMs run it, each on its own 128 rows of A and
+//   * an elected lane of one warp of the even CTA (the leader) issues tcgen05.mma.cta_group::2
+//     with M = 256, N = 256, K = 16: the tensor cores of both SMs run it, each on its own 128 rows of A and
 //     on both halves of B, and each accumulates its 128 x 256 slice in its own tensor memory;
 //   * one tcgen05.commit per event, multicast to the barrier at the same offset in both CTAs,
 //     releases a ring stage or publishes a finished accumulator in both;
@@ -20,7 +20,8 @@
 //
 // Every wait is bounded; on expiry the kernel records a code, all roles of both CTAs drain
 // (each through its own bounded waits), tensor memory is released and the kernel returns.
-// Products of more than one wave of 128x256 tiles take this kernel.  It is the CTA-pair variant of the library GEMM that torch.matmul / cuBLAS provides to the
+// Products of more than one wave of 128x256 tiles take this kernel.  It is the CTA-pair variant of
+// the library GEMM that torch.matmul / cuBLAS provides to the
 // reference trainer's nn.Linear layers (benchmarks/train_llama7b_dp_pp_lowbit.py:222-238).
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -140,8 +140,9 @@ class GPT2(torch.nn.Module):
 
     def collect_autograd_grads(self, prefix: Optional[str] = None) -> None:
         """Parameters whose gradients come from torch ops (the position embedding; LayerNorm and
-        the activation's bias without the fused ops) receive ``.grad``; fold them into the flat fp32 gradient buffer.  ``prefix`` limits the pass
-        to the parameters whose name starts with it (one layer: ``"h3."``)."""
+        the activation's bias without the fused ops) receive ``.grad``; fold them into the flat
+        fp32 gradient buffer.  ``prefix`` limits the pass to the parameters whose name starts
+        with it (one layer: ``"h3."``)."""
         want = None if prefix is None else prefix.replace(".", "_")
         for name, p in self.p.items():
             if p.grad is not None and (want is None or name.startswith(want)):

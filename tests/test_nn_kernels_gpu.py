@@ -177,8 +177,8 @@ def test_rope_backward_takes_any_alignment(offset):
 
 def test_swiglu_over_the_range_of_gates():
     """Gates from -88.5 (1 + e^-g near the largest fp32) to 88, with ups that bring the products to
-    where bf16 has its full precision.  One rounding to bf16 (8 bits: 2^-8) and an exponential that is off by
-    2 + 1.2 |g| ulp of fp32 (2^-16)."""
+    where bf16 has its full precision.  One rounding to bf16 (8 bits: 2^-8) and an exponential that
+    is off by 2 + 1.2 |g| ulp of fp32 (2^-16)."""
     g = torch.arange(-177, 177, device="cuda").double() / 2
     silu = g / (1 + torch.exp(-g))
     up = torch.exp2(-torch.floor(torch.log2(silu.abs().clamp_min(2.0 ** -122))))  # at most 2^122
